@@ -196,6 +196,7 @@ extern "C" void rwig_shutdown(void) {
     for (void* p : c->slots)
       if (p) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);
+    if (c->resident_res) cudaFreeHost(c->resident_res);
     cudaEventDestroy(c->ev0);
     cudaEventDestroy(c->ev1);
     cudaEventDestroy(c->evk);

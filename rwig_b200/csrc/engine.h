@@ -47,6 +47,10 @@ struct Context {
   std::vector<cudaEvent_t> gemm_ev;
   int gemm_ev_used = 0;
   bool gemm_timing = false;
+  // whole-solve Sinkhorn launches (sinkhorn_resident.cu): host-mapped results
+  // and the number of the last launch, which its packets' tags carry
+  double* resident_res = nullptr;
+  unsigned long long resident_epoch = 0;
   // the K whose INT8 residue planes the scratch holds (oz::prepare_reuse):
   // its size and leading dimension, valid while no other prepare ran
   bool oz_kept = false;

@@ -728,6 +728,16 @@ int sinkhorn_device(Context* ctx, cudaStream_t st, bool vanilla, double* P, doub
   const bool want_grad = withgrad && grad_a;
   double grad_ms = 0.0;
   if (want_grad && max_iter < 0) return set_error(RWIG_E_INVALID, "max_iter must be >= 0");
+  // Problems that fit on the chip run in one launch.  The log method asks for
+  // the scaling form with its default absorption bound; a problem that leaves
+  // the form's range comes back here and starts again.
+  if (vanilla || (option("log_sinkhorn.scaled", 1.0) != 0.0 && option("log_sinkhorn.tau", 100.0) >= 100.0)) {
+    int status = 0;
+    const int rc = sinkhorn_resident(ctx, st, vanilla, P, want_grad ? grad_a : nullptr, f, g, loss, iter, err, a, b, C,
+                                     M, N, reg, max_iter, zero_tol, &status);
+    if (rc < 0) return rc;
+    if (rc > 0) return status;
+  }
   int launches = 0;
 
   // support reduction (src/sinkhorn_impl_log.cpp:238-249): drop zero masses

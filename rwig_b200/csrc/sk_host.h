@@ -57,6 +57,13 @@ int sinkhorn_grad(Context* ctx, cudaStream_t st, bool vanilla, const double* C, 
                   const double* gh, int m, int n, int L, double eps, const int* ridx, int M, double out_scale,
                   double* grad_a, int* launches);
 
+// A whole solve in one launch (sinkhorn_resident.cu), grad_a optional: 1 with
+// *status and the report filled, 0 when the problem does not fit or left the
+// scaling form's range (nothing of its outputs is to be used), < 0 an error.
+int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, double* grad_a, double* f, double* g,
+                      double* loss, int* iter, double* err, const double* a, const double* b, const double* C, int M,
+                      int N, double reg, int max_iter, double zero_tol, int* status);
+
 int sinkhorn_device(Context* ctx, cudaStream_t st, bool vanilla, double* P, double* grad_a, double* f, double* g,
                     double* loss, int* iter, double* err, const double* a, const double* b, const double* C,
                     int M, int N, double reg, int withgrad, int max_iter, double zero_tol);
