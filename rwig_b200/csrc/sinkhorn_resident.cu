@@ -1,6 +1,6 @@
 // sinkhorn_resident.cu -- a whole Sinkhorn solve, vanilla or log-stabilised,
 // with or without its gradient, in one cooperative launch, for problems whose
-// kernel matrix fits on the chip (up to 4096 rows and about 29 MB).
+// kernel matrix fits on the chip (about 4 million elements).
 //
 // Both methods run in scaling form on K = exp(-C/eps):
 //   u_1 = a / (K 1),   v = b / (K^T u),   u = a / (K v)
@@ -19,25 +19,26 @@
 //   step L:  col = (pb^T 1) v / b,      ubar = (pb 1) / u - K col,
 //   step l:  col = (K^T x) v_l^2 / b,   ubar = K col,
 //   each:    grad_a += ubar u_l / a,    x = ubar u_l^2 / a.
-// So every iteration, forward or backward, is the same sweep over K.
+// So every iteration, forward or backward, is the same two passes over K.
 //
 // What bounds it: at these sizes neither memory nor arithmetic but the latency
-// of one iteration, two exchanges between CTAs plus the sweep's own barriers.
-// The general path's two grid barriers (arrive, poll), the partials read after
-// the first and the totals after the second took 13 us per iteration at every
-// size up to 2048^2.  Here:
-//   * each CTA keeps its strip of K in shared memory (its last two columns, if
-//     need be, in registers);
-//   * partial sums and totals travel as 16-byte packets (value, tag), written
-//     and read by single 128-bit accesses: a reader polls the data itself, so
-//     an exchange costs one trip through L2 instead of a fence, a counter and a
-//     second trip.  A tag holds the launch's number and the round, so packets
-//     need no reset; a round's packets are overwritten only after every reader
-//     has sent what it computed from them;
-//   * small problems use few CTAs, and each adds all partials itself (one
-//     exchange per iteration); larger ones split the rows, one warp per row;
-//   * the stopping test runs beside the next sweep's sums.
-// Measured (B200, whole calls): see the table beside launch_resident.
+// of one iteration.  With column strips, two grid barriers (arrive, poll),
+// partials read after the first and totals after the second, an iteration took
+// 13 us at every size up to 2048^2.  Here:
+//   * K is cut into gr x gc blocks, one per CTA, kept in shared memory (a few
+//     columns in registers when a block is a little too large).  A CTA needs u
+//     of its block's rows and v of its columns only, and the partial sums of a
+//     pass go to the CTAs of one block row or column: 270 numbers per CTA at
+//     1777 x 1501 where a column strip sends and receives 1777 each;
+//   * every CTA of a block row (column) adds that row's (column's) partials
+//     itself, in the same order, so totals need no second trip;
+//   * partials travel as 16-byte packets (value, tag), written and read by
+//     single 128-bit accesses: a reader polls the data itself, one trip through
+//     L2 instead of a fence, a counter and a second trip.  A tag holds the
+//     launch's number and the round, so packets need no reset;
+//   * the stopping test of an iteration runs beside the next one's column pass
+//     (whose result is thrown away when it stops).
+// The figures stand beside shape().
 #include <algorithm>
 #include <cmath>
 
@@ -49,10 +50,9 @@ namespace rwig {
 namespace skres {
 
 constexpr int NTT = 512, NW = NTT / 32;
-constexpr int kMaxRows = 4096;
-constexpr int kMaxG = 160;       // CTAs (five packets per lane of a merging warp)
-constexpr int kRowsPerWarp = 2;  // merged rows per warp: M <= 32 G
-constexpr int kRegCols = 2;      // columns of a strip that may live in registers
+constexpr int kMaxSide = 512;  // rows and columns of a block: one of each per thread
+constexpr int kMaxG = 160;     // CTAs (five error packets per lane)
+constexpr int kRegCols = 4;    // REG: columns in registers per column group of the row pass
 constexpr double kLo = 1e-250, kHi = 1e250;
 
 struct alignas(16) Packet {
@@ -66,17 +66,20 @@ struct Args {
   double* P;        // optional
   double* f;        // optional: f / u
   double* g;        // optional: g / v
-  double* grad;     // optional (with uh, vh)
-  double* uh;       // u_l at uh[l M] (l = 1..L; redundant: a copy per CTA), gradient only
-  double* vh;       // v_l at vh[l N]
+  double* grad;     // gradient: M
+  double* uh;       // gradient: u_l of each CTA's rows at [cta][l][ldm]
+  double* vh;       // gradient: v_l of each CTA's columns at [cta][l][ldn]
   const double* info;  // masses_kernel: support sizes, bad masses
-  int M, N, G, R, lds, ncmax, nsm;
-  int vanilla, redundant, max_iter;
+  int M, N, gr, gc, lds, ldm, ldn, nsm, chunks;
+  int vanilla, max_iter;
   double eps, tol;
-  Packet* part;  // redundant: [2][G][M] by the tag's parity; split: [merger][G][R]
-  Packet* up;    // [M]
-  Packet* cer;   // [2][G]
-  Packet* fin;   // [G][6]
+  // packets, two exchanges of each kind by the tag's parity: a CTA may send the
+  // next one's while a peer still reads this one's, but not the one after that,
+  // for which it needs that peer's part in the next one first
+  Packet* cpart;  // [2][gr][N] column partials
+  Packet* rpart;  // [2][gc][M] row partials
+  Packet* epart;  // [2][2][G]  error shares: rows, columns
+  Packet* fin;    // [G][6]
   unsigned long long epoch;  // launch number << 32
   double* res;               // host-mapped results (kRes*)
   unsigned* err;
@@ -87,37 +90,35 @@ __device__ __forceinline__ void put(Packet* p, double v, unsigned long long tag)
                "l"(__double_as_longlong(v)), "l"(tag)
                : "memory");
 }
-__device__ __forceinline__ bool get(const Packet* p, unsigned long long tag, double& v) {
-  unsigned long long x, t;
+__device__ __forceinline__ void get(const Packet* p, unsigned long long& v, unsigned long long& tag) {
   asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
-               : "=l"(x), "=l"(t)
+               : "=l"(v), "=l"(tag)
                : "l"(p)
                : "memory");
-  v = __longlong_as_double((long long)x);
-  return t == tag;
 }
 
-// Polls NP packets at(k), k < n, until all carry the tag; bounded (2 s, or an
-// error elsewhere).
+// Polls NP packets at(k), k < n, until all carry the tag (n <= 0: none);
+// bounded (2 s, or an error elsewhere).  All loads of a try are issued before
+// the first is looked at: a test after each load would cost a round trip to L2
+// per packet (7000-10000 clocks for a dozen, against 2000).
 template <int NP, class At>
 __device__ __forceinline__ bool poll(int n, At at, unsigned long long tag, double (&v)[NP], unsigned* err) {
-  unsigned pend = 0;
 #pragma unroll
-  for (int k = 0; k < NP; ++k) {
-    v[k] = 0.0;
-    if (k < n) pend |= 1u << k;
-  }
+  for (int k = 0; k < NP; ++k) v[k] = 0.0;
+  if (n <= 0) return true;
   unsigned long long t0 = 0;
-  for (unsigned spin = 1; pend; ++spin) {
+  for (unsigned spin = 1;; ++spin) {
+    unsigned long long x[NP], t[NP];
 #pragma unroll
-    for (int k = 0; k < NP; ++k)
-      if (pend >> k & 1u) {
-        double x;
-        if (get(at(k), tag, x)) {
-          v[k] = x;
-          pend &= ~(1u << k);
-        }
-      }
+    for (int k = 0; k < NP; ++k) get(at(k < n ? k : n - 1), x[k], t[k]);
+    bool all = true;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) all = all && t[k] == tag;
+    if (all) {
+#pragma unroll
+      for (int k = 0; k < NP; ++k) v[k] = k < n ? __longlong_as_double((long long)x[k]) : 0.0;
+      return true;
+    }
     if ((spin & 255u) == 0u) {
       if (*(volatile unsigned*)err != 0u) return false;
       const unsigned long long now = globaltimer_ns();
@@ -128,7 +129,6 @@ __device__ __forceinline__ bool poll(int n, At at, unsigned long long tag, doubl
       }
     }
   }
-  return true;
 }
 
 // Partial sums of 8 NQ columns from c0 over row pairs [p0, p1): 8 column lanes
@@ -166,534 +166,389 @@ __device__ __forceinline__ void sum_block(const double* K, int lds, int nc, int 
   }
 }
 
-// Column sums of the strip's nc shared columns with su: the 16 warps form
-// blocks of 32 columns and row chunks; red[chunk * ld + c].  Returns the chunks.
-__device__ __forceinline__ int sum_columns(const double* K, int lds, int M, int nc, int ld, const double* su, double* red) {
-  const int w = threadIdx.x >> 5;
-  const int nblk = (nc + 31) >> 5;
-  const int lg = nblk > 8 ? 4 : nblk > 4 ? 3 : nblk > 2 ? 2 : nblk > 1 ? 1 : 0;
-  const int nrc = NW >> lg, rc = w & (nrc - 1);
-  const int pairs = (M + 1) >> 1;
-  const int p0 = rc * pairs / nrc, p1 = (rc + 1) * pairs / nrc;
-  for (int blk = w >> (4 - lg); blk < nblk; blk += 1 << lg) {
-    const int c0 = 32 * blk, nq = (min(32, nc - c0) + 7) >> 3;
-    double* out = red + rc * ld;
-    if (nq == 4) sum_block<4>(K, lds, nc, c0, p0, p1, su, out);
-    else if (nq == 3) sum_block<3>(K, lds, nc, c0, p0, p1, su, out);
-    else if (nq == 2) sum_block<2>(K, lds, nc, c0, p0, p1, su, out);
-    else sum_block<1>(K, lds, nc, c0, p0, p1, su, out);
-  }
-  return nrc;
-}
-
-// Shared memory (doubles): strip [nsm][lds], su [lds], red, vs, vn, cb [ncmax]
-// each, es [4][NW], with the gradient red2 [NW][ncmax].
-__host__ __device__ constexpr int red_doubles(int ncmax) { return NW * ncmax > 1024 ? NW * ncmax : 1024; }
-__host__ __device__ constexpr size_t smem_doubles(int lds, int nsm, int ncmax, bool grad) {
-  return (size_t)nsm * lds + lds + red_doubles(ncmax) + 3 * (size_t)ncmax + 4 * NW + (grad ? NW * (size_t)ncmax : 0);
-}
-
 // Host-mapped results.
 constexpr double kResRunning = 0.0, kResFinished = 1.0, kResUnsafe = 2.0;
 enum { kResIter = 0, kResErr, kResStatus, kResLoss, kResL1Row, kResL1Col, kResL2Row, kResL2Col, kResSupM, kResSupN,
        kResKerr, kResGradNs, kResWords };
 
-// RPT rows per thread: 2 up to 1024 rows, 4 up to 2048, 8 up to 4096.  Row sets
-// of a thread: pairs 2 (lt + tg k) of the sweep's second half, and (polling u,
-// building K, the final pass) rows tid + 512 j.
-template <int RPT, bool GRAD>
+// Shared memory (doubles): block [nsm][lds], su, suo, sa [lds], sv, sd, sb
+// [ldn], colp [chunks][ldn], rowp [1024], es [8].
+__host__ __device__ constexpr size_t smem_doubles(int lds, int ldn, int nsm, int chunks) {
+  return (size_t)nsm * lds + 3 * (size_t)lds + 3 * (size_t)ldn + (size_t)chunks * ldn + 1024 + 6 * NW + 8;
+}
+
+// REG: the last kRegCols columns per column group of the row pass are held in
+// registers (nsm of the block's columns in shared memory).
+template <bool GRAD, bool REG>
 __global__ void __launch_bounds__(NTT, 1) resident_kernel(Args p) {
   extern __shared__ __align__(128) double sm[];
-  constexpr int KP = RPT / 2;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, cta = blockIdx.x;
-  const int M = p.M, N = p.N, G = p.G, lds = p.lds;
+  const int M = p.M, N = p.N, gr = p.gr, gc = p.gc, G = gr * gc, lds = p.lds, ldn = p.ldn;
+  const int ri = cta / gc, ci = cta - ri * gc;
   const double eps = p.eps, inv_eps = 1.0 / p.eps;
-  const int c0 = (int)(((long long)cta * N) / G), ncols = (int)(((long long)(cta + 1) * N) / G) - c0;
-  const int nc = min(ncols, p.nsm), nreg = ncols - nc;  // columns in shared memory, in registers
-  const int ld = p.ncmax;
+  const int m0 = (int)((long long)ri * M / gr), mr = (int)((long long)(ri + 1) * M / gr) - m0;
+  const int n0 = (int)((long long)ci * N / gc), nr = (int)((long long)(ci + 1) * N / gc) - n0;
+  const int ns = REG ? min(nr, p.nsm) : nr;  // columns in shared memory
   double* const K = sm;
   double* const su = K + (size_t)p.nsm * lds;
-  double* const red = su + lds;
-  double* const vs = red + red_doubles(ld);  // v of the last completed sweep
-  double* const vn = vs + ld;                // factors of the running sweep's second half
-  double* const cb = vn + ld;                // b
-  double* const es = cb + ld;                // [4][NW]
-  double* const red2 = es + 4 * NW;          // GRAD
-  double* const uh = GRAD ? p.uh + (p.redundant ? (size_t)cta * (p.max_iter + 2) * M : 0) : nullptr;
+  double* const suo = su + lds;  // u of the iteration before
+  double* const sa = suo + lds;
+  double* const sv = sa + lds;   // v, or the factors of the row pass
+  double* const sd = sv + ldn;   // columns' error terms
+  double* const sb = sd + ldn;
+  double* const colp = sb + ldn;
+  double* const rowp = colp + (size_t)p.chunks * ldn;
+  double* const es = rowp + 1024;
 
   if (p.info[2] != 0.0) {  // a mass the scaling form does not take, or no support
     if (cta == 0 && tid == 0) p.res[kResStatus] = kResUnsafe;
     return;
   }
-  // second half: column groups for few rows
-  const int ncg = RPT > 2 ? 1 : M <= 64 ? 16 : M <= 128 ? 8 : M <= 256 ? 4 : M <= 512 ? 2 : 1;
-  const int tg = NTT / ncg, cg = tid / tg, r0 = 2 * (tid - cg * tg);
-  int nk = 0;
-#pragma unroll
-  for (int k = 0; k < KP; ++k) nk += r0 + 2 * NTT * k < M;
+  // row pass: nrw warps cover the rows' pairs, ngrp groups of them the columns
+  const int nrw = (mr + 63) >> 6, ngrp = NW / nrw;
+  const int rw = w % nrw, grp = w / nrw;
+  const bool in_pass = grp < ngrp;
+  const int r0 = 64 * rw + 2 * lane;  // first row of this thread's pair
+  const bool row_ok = in_pass && r0 < mr;
+  double2 kr[REG ? kRegCols : 1];     // its register columns ns + grp kRegCols + q
+  const double a_i = tid < mr ? p.a[m0 + tid] : 0.0;
+  const double b_j = tid < nr ? p.b[n0 + tid] : 0.0;
+  const double rb_j = b_j != 0.0 ? 1.0 / b_j : 0.0;
+  if (tid < mr) sa[tid] = a_i;
+  if (tid < nr) sb[tid] = b_j;
+  for (int i = mr + tid; i < lds; i += NTT) su[i] = 0.0;
+  bool bad = false, ok = true;
+  // tags: the launch and the number of the exchange, counted for each kind apart
+  unsigned long long ct = p.epoch, rt = p.epoch, et = p.epoch;
 
-  // ---- K, b and the row sums of K over the support
-  double ra[RPT], uo[RPT], un[RPT];  // a, current and next u of rows tid + 512 j
-  double kr[kRegCols][RPT];          // register columns, this thread's pairs
-  bool bad = false;
-#pragma unroll
-  for (int j = 0; j < RPT; ++j) {
-    const int i = tid + j * NTT;
-    ra[j] = i < M ? p.a[i] : 0.0;
-    uo[j] = un[j] = 0.0;
-  }
-  for (int c = tid; c < ncols; c += NTT) cb[c] = p.b[c0 + c];
-  auto kernel_entry = [&](double c) {
-    const double x = exp(-c / eps);
-    if (!p.vanilla && !(x >= 2.2250738585072014e-308 && x <= 1.79e308)) bad = true;
-    return x;
-  };
-#pragma unroll 2
-  for (int c = 0; c < nc; ++c) {
-    const double* Cc = p.C + (size_t)(c0 + c) * M;
-    double* Kc = K + (size_t)c * lds;
-#pragma unroll
-    for (int j = 0; j < RPT; ++j) {
-      const int i = tid + j * NTT;
-      if (i < M) Kc[i] = kernel_entry(Cc[i]);
-    }
-  }
-  for (int c = tid; c < nc; c += NTT)
-    for (int i = M; i < lds; ++i) K[(size_t)c * lds + i] = 0.0;
-#pragma unroll
-  for (int q = 0; q < kRegCols; ++q)
-#pragma unroll
-    for (int t = 0; t < RPT; ++t) {
-      const int i = r0 + 2 * NTT * (t >> 1) + (t & 1);
-      kr[q][t] = q < nreg && i < M ? kernel_entry(p.C[(size_t)(c0 + nc + q) * M + i]) : 0.0;
-    }
-  for (int i = M + tid; i < lds; i += NTT) su[i] = 0.0;
-  __syncthreads();
-  for (int c = tid; c < ncols; c += NTT) vn[c] = cb[c] != 0.0 ? 1.0 : 0.0;
-  __syncthreads();
-
-  // ---------------------------------------------------------------- exchange
-  int row_q[RPT];  // split: packet of row r0.. in its merger's block
-  if (!p.redundant) {
-#pragma unroll
-    for (int t = 0; t < RPT; ++t) {
-      const int i = ncg > 1 ? tid : r0 + 2 * NTT * (t >> 1) + (t & 1);
-      row_q[t] = i < M ? (i / p.R * G + cta) * p.R + i % p.R : 0;
-    }
-  }
-  // A tag's partials.  Redundant merges keep two rounds: a CTA may send the next
-  // round's while another still reads this one's (of the round after that it
-  // may not: it needs that other's next partials first).  Split merges keep
-  // one: a CTA sends only after it has every row's total, and so after every
-  // merger has read its partials.
-  auto part_at = [&](unsigned long long t) { return p.part + (p.redundant && (t & 1) ? (size_t)G * M : 0); };
-  auto cer_at = [&](unsigned long long t) { return p.cer + (t & 1) * G; };
-  // The sweep's second half, r = K vn over this thread's pairs, sent as this
-  // CTA's partials of the round; extra[t] is added for the pairs (ncg = 1) or
-  // for row tid (ncg > 1, extra[0]).
-  auto send_rows = [&](unsigned long long tag, const double* extra) {
-    double r[RPT];
-#pragma unroll
-    for (int t = 0; t < RPT; ++t) r[t] = 0.0;
-    const double* col = K + (size_t)cg * lds + r0;
-    const int step = ncg * lds;
-    if (nk == KP) {
+  // K = exp(-C/eps) of the block, elements spread over the threads
+  auto build = [&]() {
+    auto entry = [&](double c) {
+      const double x = exp(-c / eps);
+      if (!p.vanilla && !(x >= 2.2250738585072014e-308 && x <= 1.79e308)) bad = true;
+      return x;
+    };
+    const int el = ns * mr;
 #pragma unroll 4
-      for (int c = cg; c < nc; c += ncg, col += step) {
-        const double v = vn[c];
+    for (int e = tid; e < el; e += NTT) {
+      const int c = e / mr, i = e - c * mr;
+      K[(size_t)c * lds + i] = entry(p.C[(size_t)(n0 + c) * M + m0 + i]);
+    }
+    for (int c = tid; c < ns; c += NTT)
+      for (int i = mr; i < lds; ++i) K[(size_t)c * lds + i] = 0.0;
+    if constexpr (REG) {
 #pragma unroll
-        for (int k = 0; k < KP; ++k) {
-          const double2 kk = *reinterpret_cast<const double2*>(col + 2 * NTT * k);
-          r[2 * k] = fma(kk.x, v, r[2 * k]);
-          r[2 * k + 1] = fma(kk.y, v, r[2 * k + 1]);
+      for (int q = 0; q < kRegCols; ++q) {
+        const int c = ns + grp * kRegCols + q;
+        const bool in = row_ok && c < nr;
+        const double* Cc = p.C + (size_t)(n0 + c) * M + m0 + r0;
+        kr[q].x = in ? entry(Cc[0]) : 0.0;
+        kr[q].y = in && r0 + 1 < mr ? entry(Cc[1]) : 0.0;
+      }
+    }
+  };
+  // Row pass: partial sums over the block's columns of K sv -> rowp[grp][mr].
+  auto row_pass = [&]() {
+    double x = 0.0, y = 0.0;
+    if (row_ok) {
+      const double* col = K + (size_t)grp * lds + r0;
+      const int step = ngrp * lds;
+#pragma unroll 8
+      for (int c = grp; c < ns; c += ngrp, col += step) {
+        const double2 kk = *reinterpret_cast<const double2*>(col);
+        const double v = sv[c];
+        x = fma(kk.x, v, x);
+        y = fma(kk.y, v, y);
+      }
+      if constexpr (REG) {
+#pragma unroll
+        for (int q = 0; q < kRegCols; ++q) {
+          const int c = ns + grp * kRegCols + q;
+          const double v = c < nr ? sv[c] : 0.0;
+          x = fma(kr[q].x, v, x);
+          y = fma(kr[q].y, v, y);
         }
       }
-    } else {
-      for (int c = cg; c < nc; c += ncg, col += step) {
-        const double v = vn[c];
-#pragma unroll
-        for (int k = 0; k < KP - 1; ++k)
-          if (k < nk) {
-            const double2 kk = *reinterpret_cast<const double2*>(col + 2 * NTT * k);
-            r[2 * k] = fma(kk.x, v, r[2 * k]);
-            r[2 * k + 1] = fma(kk.y, v, r[2 * k + 1]);
-          }
-      }
+      rowp[grp * mr + r0] = x;
+      if (r0 + 1 < mr) rowp[grp * mr + r0 + 1] = y;
     }
-    if (cg == 0)
-#pragma unroll
-      for (int q = 0; q < kRegCols; ++q)
-        if (q < nreg)
-#pragma unroll
-          for (int t = 0; t < RPT; ++t) r[t] = fma(kr[q][t], vn[nc + q], r[t]);
-    if (ncg > 1) {  // the groups' sums in group order, then one row per thread
-      __syncthreads();
-      if (r0 < M) red[cg * M + r0] = r[0];
-      if (r0 + 1 < M) red[cg * M + r0 + 1] = r[1];
-      __syncthreads();
-      if (tid < M) {
-        double s = 0.0;
-        for (int q = 0; q < ncg; ++q) s += red[q * M + tid];
-        if (extra) s = extra[0] - s;
-        put(p.redundant ? part_at(tag) + (size_t)cta * M + tid : p.part + row_q[0], s, tag);
-      }
-    } else {
-#pragma unroll
-      for (int t = 0; t < RPT; ++t) {
-        const int i = r0 + 2 * NTT * (t >> 1) + (t & 1);
-        if (i < M) put(p.redundant ? part_at(tag) + (size_t)cta * M + i : p.part + row_q[t], extra ? extra[t] - r[t] : r[t], tag);
-      }
-    }
+    __syncthreads();
   };
-  // Totals of the round's partials -> x_i = fn(i, j, total) for rows tid + 512 j
-  // into `out` (every CTA gets all rows).  fn runs once per row and CTA
-  // (redundant; j: its index here) or once per row on its merger (j = -1, slot
-  // = the merger's row of this warp).
-  const int q0 = cta * p.R, q1 = min(M, q0 + p.R);  // split: this CTA's rows
-  auto totals = [&](unsigned long long tag, double (&out)[RPT], auto fn) -> bool {
-    bool ok = true;
-    if (p.redundant) {
-#pragma unroll
-      for (int j = 0; j < RPT; ++j) {
-        const int i = tid + j * NTT;
-        if (i >= M) continue;
-        double acc = 0.0;
-        for (int k = 0; k < G && ok; k += 8) {
-          double x[8];
-          ok = poll<8>(min(8, G - k), [&](int e) { return part_at(tag) + (size_t)(k + e) * M + i; }, tag, x, p.err);
-#pragma unroll
-          for (int e = 0; e < 8; ++e)
-            if (k + e < G) acc += x[e];
-        }
-        out[j] = fn(i, j, acc);
-      }
-      return ok;
-    }
-#pragma unroll
-    for (int s = 0; s < kRowsPerWarp; ++s) {
-      const int i = q0 + w + NW * s;
-      if (i < q1) {  // warp-uniform
-        constexpr int NP = kMaxG / 32;
-        double x[NP];
-        const Packet* base = p.part + (size_t)cta * G * p.R + (i - q0);
-        const int n = (G - lane + 31) >> 5;
-        ok = poll<NP>(n, [&](int e) { return base + (size_t)(lane + 32 * e) * p.R; }, tag, x, p.err) && ok;
-        double t = 0.0;
-#pragma unroll
-        for (int e = 0; e < NP; ++e) t += x[e];
-        t = warp_sum(t);
-        if (lane == 0) put(p.up + i, fn(i, -1 - s, t), tag);
-      }
-    }
-    double x[RPT];
-    const int n = tid < M ? (M - tid + NTT - 1) / NTT : 0;
-    ok = poll<RPT>(n, [&](int j) { return p.up + tid + j * NTT; }, tag, x, p.err) && ok;
-#pragma unroll
-    for (int j = 0; j < RPT; ++j) out[j] = x[j];
-    return ok;
-  };
-  auto store_su = [&](const double (&x)[RPT]) {
-#pragma unroll
-    for (int j = 0; j < RPT; ++j)
-      if (tid + j * NTT < M) su[tid + j * NTT] = x[j];
-  };
-  // Column sums of the whole strip with su: red[chunk * ld + c], chunks returned
-  // (register columns: NW warps' partials).
-  auto sums = [&]() {
-    const int n = sum_columns(K, lds, M, nc, ld, su, red);
-    if (nreg > 0) {
-      double u[RPT];
-#pragma unroll
-      for (int t = 0; t < RPT; ++t) {
-        const int i = r0 + 2 * NTT * (t >> 1) + (t & 1);
-        u[t] = i < M ? su[i] : 0.0;
-      }
-#pragma unroll
-      for (int q = 0; q < kRegCols; ++q)
-        if (q < nreg) {
-          double x = 0.0;
-#pragma unroll
-          for (int t = 0; t < RPT; ++t) x = fma(kr[q][t], u[t], x);
-          x = warp_sum(cg == 0 ? x : 0.0);
-          if (lane == 0) red[w * ld + nc + q] = x;
-        }
-    }
-    return n;
-  };
-  auto col_total = [&](int c, int n) {
-    double x[NW];
-    const int m = c < nc ? n : NW;
-#pragma unroll
-    for (int q = 0; q < NW; ++q) x[q] = q < m ? red[q * ld + c] : 0.0;
-#pragma unroll
-    for (int h = NW / 2; h >= 1; h >>= 1)
-#pragma unroll
-      for (int q = 0; q < h; ++q) x[q] += x[q + h];
-    return x[0];
-  };
-  auto sum_es = [&](int k) {
+  // The rows' totals over the block row (thread tid < mr: row m0 + tid): this
+  // CTA's partial (`extra` minus it, when given) sent and all gc added in order.
+  auto row_total = [&](const double* extra) {
     double t = 0.0;
+    const unsigned long long tag = ++rt;
+    if (tid < mr) {
+      for (int q = 0; q < ngrp; ++q) t += rowp[q * mr + tid];
+      if (extra) t = *extra - t;
+      if (gc > 1) {
+        Packet* base = p.rpart + (tag & 1) * (size_t)gc * M + m0 + tid;
+        put(base + (size_t)ci * M, t, tag);
+        t = 0.0;
+        for (int k = 0; k < gc && ok; k += 12) {
+          double x[12];
+          ok = poll<12>(min(12, gc - k), [&](int e) { return base + (size_t)(k + e) * M; }, tag, x, p.err);
 #pragma unroll
-    for (int q = 0; q < NW; ++q) t += es[k * NW + q];
+          for (int e = 0; e < 12; ++e) t += x[e];
+        }
+      }
+    }
+    return t;
+  };
+  // Column pass: partial sums over the block's rows of K^T su -> colp[chunk][ldn];
+  // returns the chunks (register columns: nrw).
+  const int nblk = (p.nsm + 31) >> 5;  // (the same in every CTA: it sizes colp)
+  const int lg = nblk > 8 ? 4 : nblk > 4 ? 3 : nblk > 2 ? 2 : nblk > 1 ? 1 : 0;
+  const int nrc = NW >> lg;
+  const int pairs = (mr + 1) >> 1;
+  const int p0 = (w & (nrc - 1)) * pairs >> (4 - lg), p1 = ((w & (nrc - 1)) + 1) * pairs >> (4 - lg);
+  auto col_pass = [&]() {
+    for (int blk = w >> (4 - lg); blk < nblk; blk += 1 << lg) {
+      const int c0 = 32 * blk, nq = (min(32, ns - c0) + 7) >> 3;
+      double* out = colp + (w & (nrc - 1)) * ldn;
+      if (nq == 4) sum_block<4>(K, lds, ns, c0, p0, p1, su, out);
+      else if (nq == 3) sum_block<3>(K, lds, ns, c0, p0, p1, su, out);
+      else if (nq == 2) sum_block<2>(K, lds, ns, c0, p0, p1, su, out);
+      else sum_block<1>(K, lds, ns, c0, p0, p1, su, out);
+    }
+    if constexpr (REG) {
+      const double u0 = row_ok ? su[r0] : 0.0, u1 = row_ok ? su[r0 + 1] : 0.0;
+#pragma unroll
+      for (int q = 0; q < kRegCols; ++q) {
+        const double x = warp_sum(fma(kr[q].x, u0, kr[q].y * u1));
+        const int c = ns + grp * kRegCols + q;
+        if (lane == 0 && in_pass && c < nr) colp[rw * ldn + c] = x;
+      }
+    }
+    __syncthreads();
+  };
+  // The columns' totals over the block column (thread tid < nr: column n0 + tid).
+  auto col_total = [&]() {
+    double t = 0.0;
+    const unsigned long long tag = ++ct;
+    if (tid < nr) {
+      const int n = REG && tid >= ns ? nrw : nrc;
+      for (int q = 0; q < n; ++q) t += colp[q * ldn + tid];
+      if (gr > 1) {
+        Packet* base = p.cpart + (tag & 1) * (size_t)gr * N + n0 + tid;
+        put(base + (size_t)ri * N, t, tag);
+        t = 0.0;
+        for (int k = 0; k < gr && ok; k += 12) {
+          double x[12];
+          ok = poll<12>(min(12, gr - k), [&](int e) { return base + (size_t)(k + e) * N; }, tag, x, p.err);
+#pragma unroll
+          for (int e = 0; e < 12; ++e) t += x[e];
+        }
+      }
+    }
     return t;
   };
   auto in_range = [](double x) { return x >= kLo && x <= kHi; };
-  // u_{l} = a / total
-  double ga[RPT];        // gradient (redundant: rows tid + 512 j; split: [s] the merger's rows, lane 0)
+  double* const uh = GRAD ? p.uh + (size_t)cta * (p.max_iter + 2) * p.ldm : nullptr;
+  double* const vh = GRAD ? p.vh + (size_t)cta * (p.max_iter + 2) * ldn : nullptr;
+  // Sum over CTAs of error share q of exchange et, by one warp.
+  auto error_at = [&](int q) { return p.epart + ((et & 1) * 2 + q) * G; };
+  auto error_sum = [&](int q) {
+    double x[kMaxG / 32], t = 0.0;
+    const Packet* base = error_at(q);
+    const unsigned long long tag = et;
+    ok = poll<kMaxG / 32>((G - lane + 31) >> 5, [&](int k) { return base + lane + 32 * k; }, tag, x, p.err) && ok;
 #pragma unroll
-  for (int j = 0; j < RPT; ++j) ga[j] = 0.0;
-  auto next_u = [&](int l) {
-    return [&, l](int i, int j, double t) {
-      const double a = j >= 0 ? ra[j >= 0 ? j : 0] : p.a[i];
-      // a total outside the safe range ends the solve (its u is checked by every CTA)
-      const double u = a == 0.0 ? 0.0 : in_range(t) ? a / t : INFINITY;
-      if (GRAD) uh[(size_t)l * M + i] = u;
-      return u;
-    };
+    for (int k = 0; k < kMaxG / 32; ++k) t += x[k];
+    return warp_sum(t);
   };
+
   // ---------------------------------------------------------------- forward
-  unsigned long long tag = p.epoch + 1;
-  {
-    const double nb = __syncthreads_or(bad) ? INFINITY : 0.0;
-    if (tid == 0) put(cer_at(tag) + cta, nb, tag);
+  build();
+  if (tid < nr) {
+    sv[tid] = b_j != 0.0 ? 1.0 : 0.0;  // K 1 over the support
+    sd[tid] = 0.0;
   }
-  send_rows(tag, nullptr);
+  bad = __syncthreads_or(bad);
+  // each CTA's share of the error: rows and columns of its block's row and column
+  const int ea = ci * mr / gc, eb = (ci + 1) * mr / gc, ec0 = ri * nr / gr, ec1 = (ri + 1) * nr / gr;
   int iter = 0;
-  double status = kResRunning;
-  double err = 1000.0;
-  bool ok = true;
+  double err = 1000.0, u = 1.0, v = 0.0, vo = 0.0;
+  row_pass();
+  u = row_total(nullptr);
+  // iteration k = iter + 1: u_k from the totals, v_k, totals of K v_k
   while (true) {
-    // u of the next iteration, and (beside its sums) the error of the last one
-    ok = totals(tag, un, next_u(iter + 1));
-    store_su(un);
+    const double uo = iter > 0 ? su[tid < mr ? tid : 0] : 0.0;
+    u = a_i == 0.0 ? 0.0 : in_range(u) ? a_i / u : INFINITY;  // (an infinite u fails the range check below)
+    if (tid < mr) {
+      suo[tid] = uo;
+      su[tid] = u;
+      if (GRAD) uh[(size_t)(iter + 1) * p.ldm + tid] = u;
+    }
     if (__syncthreads_or(!ok)) {
       ok = false;
       break;
     }
-    const int n = sums();
-    {
-      double e = 0.0;
-#pragma unroll
-      for (int j = 0; j < RPT; ++j) {
-        if (tid + j * NTT >= M || ra[j] == 0.0) continue;
-        if (!in_range(un[j])) e = INFINITY;
+    ++et;
+    if (w == NW - 1) {  // this CTA's share of the last iteration's error (of iteration 0: the range checks)
+      double e = bad ? INFINITY : 0.0, ec = 0.0;
+      for (int i = ea + lane; i < eb; i += 32) {
+        const double a = sa[i], x = su[i];
+        if (a == 0.0) continue;
+        if (!in_range(x)) e = INFINITY;
         else if (iter > 0) {
-          const double q = uo[j] / un[j];  // u_i (K v)_i / a_i
-          const double d = p.vanilla ? ra[j] * (q - 1.0) : log(q);
+          const double q = suo[i] / x;  // u_i (K v)_i / a_i
+          const double d = p.vanilla ? a * (q - 1.0) : log(q);
           e = fma(d, d, e);
         }
       }
+      for (int c = ec0 + lane; c < ec1; c += 32) ec += sd[c];
       e = warp_sum(e);
-      if (lane == 0) es[w] = e;
-      if (w == NW - 1) {
-        double x[kMaxG / 32], t = 0.0;
-        ok = poll<kMaxG / 32>((G - lane + 31) >> 5, [&](int k) { return cer_at(tag) + lane + 32 * k; }, tag, x, p.err);
-#pragma unroll
-        for (int k = 0; k < kMaxG / 32; ++k) t += x[k];
-        t = warp_sum(t);
-        if (lane == 0) es[NW] = t;
+      ec = warp_sum(ec);
+      if (lane < 2) put(error_at(lane) + cta, lane ? ec : e, et);
+    }
+    col_pass();
+    const double s = col_total();
+    if (w == NW - 1) {
+      const double e0 = error_sum(0), e1 = error_sum(1);
+      if (lane == 0) {
+        const double e = sqrt(e0) + sqrt(e1);
+        es[0] = e;
+        es[1] = !(e0 + e1 <= 1e300) ? 2.0 : iter > 0 && !(iter < p.max_iter && e >= p.tol) ? 1.0 : 0.0;
       }
     }
+    vo = v;
+    v = b_j / s;
+    if (b_j == 0.0) v = 0.0;
+    __syncthreads();  // (the row pass and the error share have read sv and sd)
+    if (es[1] != 0.0) break;
+    if (tid < nr) {
+      sv[tid] = v;
+      const double d = p.vanilla ? fma(v, s, -b_j) : fma(v, s, -b_j) * rb_j;  // log(v s / b) to first order
+      sd[tid] = b_j == 0.0 ? 0.0 : in_range(s) && in_range(v) ? d * d : INFINITY;
+      if (GRAD) vh[(size_t)(iter + 1) * ldn + tid] = v;
+    }
+    ++iter;
     if (__syncthreads_or(!ok)) {
       ok = false;
       break;
     }
-    const double er = sum_es(0), ec = es[NW];
-    if (!(er + ec <= 1e300)) {
-      status = kResUnsafe;
-      break;
-    }
-    if (iter > 0) {
-      err = sqrt(er) + sqrt(ec);
-      if (!(iter < p.max_iter && err >= p.tol)) break;
-    }
-    ++iter;
-    ++tag;
-    // v = b / (K^T u)
-    double e = 0.0;
-    for (int c = tid; c < ncols; c += NTT) {
-      const double b = cb[c], s = col_total(c, n);
-      const double v = b / s;
-      vn[c] = b == 0.0 ? 0.0 : v;
-      vs[c] = vn[c];
-      if (GRAD) p.vh[(size_t)iter * N + c0 + c] = vn[c];
-      if (b != 0.0) {
-        const double d = p.vanilla ? fma(v, s, -b) : fma(v, s, -b) / b;  // log(v s / b) to first order
-        e = in_range(s) && in_range(v) ? fma(d, d, e) : INFINITY;
-      }
-    }
-    e = warp_sum(e);
-    if (lane == 0) es[2 * NW + w] = e;
-#pragma unroll
-    for (int j = 0; j < RPT; ++j) uo[j] = un[j];
-    __syncthreads();
-    if (tid == 0) put(cer_at(tag) + cta, sum_es(2), tag);
-    send_rows(tag, nullptr);
+    row_pass();
+    u = row_total(nullptr);
   }
-  if (!ok || status == kResUnsafe) {
+  ok = !__syncthreads_or(!ok);
+  if (!ok || es[1] == 2.0) {
     if (cta == 0 && tid == 0) {
       p.res[kResKerr] = ok ? 0.0 : 1.0;
       p.res[kResStatus] = kResUnsafe;
     }
     return;
   }
+  err = es[0];
+  u = tid < mr ? suo[tid] : 0.0;  // the stopped iteration's scalings
+  v = vo;
 
   // ---------------------------------------------------------------- plan, loss, marginals
-  ++tag;
-  double f[RPT], pr[RPT], rp[RPT];  // f, row sums of P and of pb, rows tid + 512 j
-  double l1 = 0.0, l2 = 0.0, cl1 = 0.0, cl2 = 0.0;
-#pragma unroll
-  for (int j = 0; j < RPT; ++j) {
-    const int i = tid + j * NTT;
-    f[j] = eps * log(uo[j]);
-    pr[j] = rp[j] = 0.0;
-    if (cta == 0 && i < M && p.f) p.f[i] = p.vanilla ? uo[j] : f[j];
+  const double fi = eps * log(u), gj = eps * log(v);
+  __syncthreads();
+  if (tid < mr) {
+    su[tid] = fi;
+    if (ci == 0 && p.f) p.f[m0 + tid] = p.vanilla ? u : fi;
   }
-  __syncthreads();  // vn, red are free
-  for (int c = tid; c < ncols; c += NTT) {
-    const double gj = eps * log(vs[c]);
-    vn[c] = gj;
-    if (p.g) p.g[c0 + c] = p.vanilla ? vs[c] : gj;
+  if (tid < nr) {
+    sd[tid] = gj;
+    if (ri == 0 && p.g) p.g[n0 + tid] = p.vanilla ? v : gj;
   }
   __syncthreads();
+  double l1 = 0.0, l2 = 0.0;
   bool zero_plan = false;
-  for (int cc = 0; cc < ncols; cc += 4) {
-    double cs[4], cp[4];
+  // P (pass 0) or pb = (C + eps log P) o P (pass 1) in K's place
+  auto plan = [&](int pass) {
+    auto entry = [&](double c, int i, int j) {
+      if (sa[i] == 0.0 || sb[j] == 0.0) return 0.0;
+      const double x = -((c - su[i]) - sd[j]) * inv_eps;
+      const double pv = exp(x);
+      // log P: x itself, which exp's rounding moves by less than one unit of
+      // the last place of 1; minus infinity where P underflowed
+      const double lp = pv > 0.0 ? x : -INFINITY;
+      if (pass == 0) {
+        l1 += c * pv;
+        l2 += pv * (lp - 1.0);
+        zero_plan |= !(pv > 0.0);
+      }
+      return pass == 0 ? pv : (c + eps * lp) * pv;
+    };
+    const int el = ns * mr;
+#pragma unroll 2
+    for (int e = tid; e < el; e += NTT) {
+      const int c = e / mr, i = e - c * mr;
+      const size_t at = (size_t)(n0 + c) * M + m0 + i;
+      const double x = entry(p.C[at], i, c);
+      K[(size_t)c * lds + i] = x;
+      if (pass == 0 && p.P) p.P[at] = x;
+    }
+    if constexpr (REG) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      cs[q] = cp[q] = 0.0;
-      const int c = cc + q;
-      if (c >= ncols) continue;
-      const bool live = cb[c] != 0.0;
-      const double gj = vn[c];
-      const double* Cc = p.C + (size_t)(c0 + c) * M;
-#pragma unroll
-      for (int j = 0; j < RPT; ++j) {
-        const int i = tid + j * NTT;
-        if (i >= M) continue;
-        double pv = 0.0;
-        if (live && ra[j] != 0.0) {
-          const double cij = Cc[i];
-          pv = exp(-((cij - f[j]) - gj) * inv_eps);
-          const double lp = log(pv);
-          l1 += cij * pv;
-          l2 += pv * (lp - 1.0);
-          pr[j] += pv;
-          cs[q] += pv;
-          if (GRAD) {
-            const double pb = (cij + eps * lp) * pv;
-            rp[j] += pb;
-            cp[q] += pb;
-            zero_plan |= !(pv > 0.0);
-          }
+      for (int q = 0; q < kRegCols; ++q) {
+        const int c = ns + grp * kRegCols + q;
+        if (!(row_ok && c < nr)) continue;
+        const size_t at = (size_t)(n0 + c) * M + m0 + r0;
+        kr[q].x = entry(p.C[at], r0, c);
+        if (pass == 0 && p.P) p.P[at] = kr[q].x;
+        if (r0 + 1 < mr) {
+          kr[q].y = entry(p.C[at + 1], r0 + 1, c);
+          if (pass == 0 && p.P) p.P[at + 1] = kr[q].y;
         }
-        if (p.P) p.P[(size_t)(c0 + c) * M + i] = pv;
       }
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (cc + q >= ncols) continue;
-      double t = warp_sum(cs[q]);
-      if (lane == 0) red[w * ld + cc + q] = t;
-      if (GRAD) {
-        t = warp_sum(cp[q]);
-        if (lane == 0) red2[w * ld + cc + q] = t;
-      }
-    }
-  }
-  __syncthreads();
-  for (int c = tid; c < ncols; c += NTT) {
-    double t = 0.0;
-    for (int q = 0; q < NW; ++q) t += red[q * ld + c];
-    if (cb[c] != 0.0) {
-      cl1 += fabs(t - cb[c]);
-      cl2 += (t - cb[c]) * (t - cb[c]);
-    }
-    if (GRAD) {  // col of step L
-      t = 0.0;
-      for (int q = 0; q < NW; ++q) t += red2[q * ld + c];
-      vn[c] = cb[c] != 0.0 ? t * vs[c] / cb[c] : 0.0;
-    }
-  }
-  // row sums of P to their mergers (redundant: to CTA 0)
-#pragma unroll
-  for (int j = 0; j < RPT; ++j) {
-    const int i = tid + j * NTT;
-    if (i < M) put(part_at(tag) + (p.redundant ? (size_t)cta * M + i : (size_t)(i / p.R * G + cta) * p.R + i % p.R), pr[j], tag);
-  }
-  double a1 = 0.0, a2 = 0.0;
-  auto row_marginal = [&](int i, double t) {
-    const double a = p.a[i];
-    if (a != 0.0) {
-      a1 += fabs(t - a);
-      a2 += (t - a) * (t - a);
-    }
-  };
-  if (p.redundant) {
-    if (cta == 0)
-#pragma unroll
-      for (int j = 0; j < RPT; ++j) {
-        const int i = tid + j * NTT;
-        if (i >= M) continue;
-        double acc = 0.0;
-        for (int k = 0; k < G && ok; ++k) {
-          double x[1];
-          ok = poll<1>(1, [&](int) { return part_at(tag) + (size_t)k * M + i; }, tag, x, p.err);
-          acc += x[0];
-        }
-        row_marginal(i, acc);
-      }
-  } else {
-#pragma unroll
-    for (int s = 0; s < kRowsPerWarp; ++s) {
-      const int i = q0 + w + NW * s;
-      if (i < q1) {
-        constexpr int NP = kMaxG / 32;
-        double x[NP], t = 0.0;
-        const Packet* base = p.part + (size_t)cta * G * p.R + (i - q0);
-        ok = poll<NP>((G - lane + 31) >> 5, [&](int e) { return base + (size_t)(lane + 32 * e) * p.R; }, tag, x, p.err) && ok;
-#pragma unroll
-        for (int e = 0; e < NP; ++e) t += x[e];
-        t = warp_sum(t);
-        if (lane == 0) row_marginal(i, t);
-      }
-    }
-  }
-  // block sums of the six scalars, sent to CTA 0
-  {
-    double v[6] = {l1, l2, cl1, cl2, a1, a2};
     __syncthreads();
+  };
+  // row and column sums of what stands in K's place (su, sv: ones)
+  auto margins = [&](double& row, double& col) {
+    if (tid < mr) su[tid] = 1.0;
+    if (tid < nr) sv[tid] = 1.0;
+    __syncthreads();
+    col_pass();
+    col = col_total();
+    row_pass();
+    row = row_total(nullptr);
+    __syncthreads();
+  };
+  double row = 0.0, col = 0.0;
+  plan(0);
+  margins(row, col);
+  {
+    const bool ra = ci == 0 && tid < mr && a_i != 0.0, cb = ri == 0 && tid < nr && b_j != 0.0;
+    const double dr = ra ? row - a_i : 0.0, dc = cb ? col - b_j : 0.0;
+    const double t6[6] = {l1, l2, fabs(dc), dc * dc, fabs(dr), dr * dr};
 #pragma unroll
     for (int t = 0; t < 6; ++t) {
-      const double x = warp_sum(v[t]);
-      if (lane == 0) red[t * NW + w] = x;
+      const double x = warp_sum(t6[t]);
+      if (lane == 0) rowp[t * NW + w] = x;
     }
     const bool zp = __syncthreads_or(zero_plan);
     if (tid < 6) {
       double t = 0.0;
-      for (int q = 0; q < NW; ++q) t += red[tid * NW + q];
-      put(p.fin + cta * 6 + tid, t, tag);
+      for (int q = 0; q < NW; ++q) t += rowp[tid * NW + q];
+      put(p.fin + cta * 6 + tid, t, p.epoch);
     }
-    if (GRAD && tid == 0) put(cer_at(tag) + cta, zp ? INFINITY : 0.0, tag);  // (its row marginals are merged)
+    ++et;
+    if (GRAD && tid == 0) put(error_at(0) + cta, zp ? INFINITY : 0.0, et);
   }
   if (cta == 0) {
     if (w < 6) {
       double x[kMaxG / 32], t = 0.0;
-      ok = poll<kMaxG / 32>((G - lane + 31) >> 5, [&](int k) { return p.fin + (lane + 32 * k) * 6 + w; }, tag, x, p.err) && ok;
+      ok = poll<kMaxG / 32>((G - lane + 31) >> 5, [&](int k) { return p.fin + (lane + 32 * k) * 6 + w; }, p.epoch, x, p.err) && ok;
 #pragma unroll
       for (int k = 0; k < kMaxG / 32; ++k) t += x[k];
       t = warp_sum(t);
-      if (lane == 0) es[w] = t;
+      if (lane == 0) es[2 + w] = t;
     }
-    ok = !__syncthreads_or(!ok);
+    ok = !__syncthreads_or(!ok || *(volatile unsigned*)p.err != 0u);
     if (tid == 0) {
       p.res[kResIter] = iter;
       p.res[kResErr] = err;
-      p.res[kResLoss] = es[0] + eps * es[1];
-      p.res[kResL1Row] = es[4];
-      p.res[kResL1Col] = es[2];
-      p.res[kResL2Row] = sqrt(es[5]);
-      p.res[kResL2Col] = sqrt(es[3]);
+      p.res[kResLoss] = es[2] + eps * es[3];
+      p.res[kResL1Row] = es[6];
+      p.res[kResL1Col] = es[4];
+      p.res[kResL2Row] = sqrt(es[7]);
+      p.res[kResL2Col] = sqrt(es[5]);
       p.res[kResSupM] = p.info[0];
       p.res[kResSupN] = p.info[1];
       p.res[kResGradNs] = 0.0;
@@ -707,81 +562,48 @@ __global__ void __launch_bounds__(NTT, 1) resident_kernel(Args p) {
     // a plan entry that underflowed: the reference's sums turn NaN or infinite
     // there, which the general path reproduces
     if (w == 0) {
-      double x[kMaxG / 32], t = 0.0;
-      ok = poll<kMaxG / 32>((G - lane + 31) >> 5, [&](int k) { return cer_at(tag) + lane + 32 * k; }, tag, x, p.err) && ok;
-#pragma unroll
-      for (int k = 0; k < kMaxG / 32; ++k) t += x[k];
-      t = warp_sum(t);
-      if (lane == 0) es[3 * NW] = t;
+      const double t = error_sum(0);
+      if (lane == 0) es[1] = t;
     }
     ok = !__syncthreads_or(!ok);
-    if (!ok || !(es[3 * NW] <= 1e300)) {
+    if (!ok || !(es[1] <= 1e300)) {
       if (cta == 0 && tid == 0) {
         p.res[kResKerr] = ok ? 0.0 : 1.0;
         p.res[kResStatus] = kResUnsafe;
       }
       return;
     }
-    // step L: this CTA's share of (pb 1) / u rides along
-#pragma unroll
-    for (int j = 0; j < RPT; ++j) {
-      const int i = tid + j * NTT;
-      if (i < M) su[i] = ra[j] != 0.0 ? rp[j] / uo[j] : 0.0;
-    }
+    if (tid < mr) su[tid] = fi;
     __syncthreads();
-    double ex[RPT];
-#pragma unroll
-    for (int t = 0; t < RPT; ++t) {
-      const int i = ncg > 1 ? tid : r0 + 2 * NTT * (t >> 1) + (t & 1);
-      ex[t] = i < M ? su[i] : 0.0;
-    }
-    ++tag;
-    send_rows(tag, ex);
-    double x[RPT];
+    plan(1);
+    margins(row, col);
+    build();
+    if (tid < nr) sv[tid] = b_j != 0.0 ? col * v * rb_j : 0.0;
+    // (pb 1) / u: the whole row total here, so one CTA of the block row brings it in
+    const double ex = ci == 0 && a_i != 0.0 ? row / u : 0.0;
+    __syncthreads();
+    row_pass();
+    double t = row_total(&ex), ga = 0.0;
     for (int l = iter;; --l) {
-      // x = ubar u_l^2 / a, grad += ubar u_l / a
-      ok = totals(tag, x, [&](int i, int j, double t) {
-        const double a = j >= 0 ? ra[j >= 0 ? j : 0] : p.a[i];
-        if (a == 0.0) return 0.0;
-        const double u = uh[(size_t)l * M + i];  // written by this thread
-        const double q = t * u / a;
-        if (j >= 0) ga[j >= 0 ? j : 0] += q;
-        else ga[j < 0 ? -1 - j : 0] += q;
-        return q * u;
-      });
-      if (l == 1) {
-        ok = !__syncthreads_or(!ok);
-        break;
-      }
-      store_su(x);
-      double vl = 0.0;
-      if (tid < ncols) vl = __ldcg(p.vh + (size_t)(l - 1) * N + c0 + tid);
+      const double ul = tid < mr && a_i != 0.0 ? uh[(size_t)l * p.ldm + tid] : 0.0;  // written by this thread
+      const double q = a_i != 0.0 ? t * ul / a_i : 0.0;
+      ga += q;
+      if (l == 1) break;
+      const double vl = tid < nr ? vh[(size_t)(l - 1) * ldn + tid] : 0.0;
+      if (tid < mr) su[tid] = q * ul;
       if (__syncthreads_or(!ok)) {
         ok = false;
         break;
       }
-      const int n = sums();
+      col_pass();
+      const double s = col_total();
+      if (tid < nr) sv[tid] = s * (vl * vl) * rb_j;
       __syncthreads();
-      for (int c = tid; c < ncols; c += NTT) {
-        const double v = c < NTT ? vl : __ldcg(p.vh + (size_t)(l - 1) * N + c0 + c);
-        vn[c] = cb[c] != 0.0 ? col_total(c, n) * (v * v) / cb[c] : 0.0;
-      }
-      __syncthreads();
-      ++tag;
-      send_rows(tag, nullptr);
+      row_pass();
+      t = row_total(nullptr);
     }
-    if (p.redundant) {
-      if (cta == 0)
-#pragma unroll
-        for (int j = 0; j < RPT; ++j)
-          if (tid + j * NTT < M) p.grad[tid + j * NTT] = ga[j];
-    } else {
-#pragma unroll
-      for (int s = 0; s < kRowsPerWarp; ++s) {
-        const int i = q0 + w + NW * s;
-        if (i < q1 && lane == 0) p.grad[i] = ga[s];
-      }
-    }
+    if (ci == 0 && tid < mr) p.grad[m0 + tid] = ga;
+    ok = !__syncthreads_or(!ok || *(volatile unsigned*)p.err != 0u);
     if (cta == 0 && tid == 0) {
       p.res[kResGradNs] = (double)(globaltimer_ns() - t_b);
       p.res[kResKerr] = ok ? 0.0 : 1.0;
@@ -819,59 +641,66 @@ __global__ void __launch_bounds__(NTT) masses_kernel(const double* a, const doub
   }
 }
 
-// Leading dimension of a shared strip: ldk / 2 odd, so that the 16-byte loads
-// of eight neighbouring columns hit all banks.
-int strip_ld(int M) {
-  const int e = (M + 1) & ~1;
-  return (e >> 1) & 1 ? e : e + 2;
-}
-
 struct Shape {
-  int G, R, lds, ncmax, nsm, redundant;
+  int gr, gc, lds, ldm, ldn, nsm, chunks, reg;
   size_t smem;
 };
 
-// The launch of an M x N problem; false when it does not fit.
-//
-// G: 8192 elements (64 KB) of K per CTA, up to every SM: below that a sweep
-// takes about 1 us, no longer than the exchange that more CTAs would lengthen.
-// Redundant merges while a CTA adds at most 4096 partials (8 per thread).
-bool shape(const Context* ctx, int M, int N, bool grad, Shape* s) {
-  if (M > kMaxRows || ctx->sm_count > kMaxG) return false;
-  const int gmax = std::min(N, ctx->sm_count);
-  const long long el = (long long)M * N;
-  int G = (int)std::min<long long>(gmax, std::max<long long>(1, (el + 8191) / 8192));
-  s->lds = strip_ld(M);
-  for (; G <= gmax; ++G) {
-    s->ncmax = (N + G - 1) / G;
-    const size_t fixed = smem_doubles(s->lds, 0, s->ncmax, grad) * 8;
-    if (fixed >= (size_t)ctx->smem_optin) continue;
-    const int room = (int)(((size_t)ctx->smem_optin - fixed) / (8 * (size_t)s->lds));
-    s->nsm = std::min(s->ncmax, room);
-    if (s->nsm < 1 || s->ncmax - s->nsm > kRegCols) continue;
-    s->R = (M + G - 1) / G;
-    s->redundant = (long long)G * M <= 4096;
-    if (!s->redundant && s->R > NW * kRowsPerWarp) {  // more rows than a merger's warps take
-      if (M <= NW * kRowsPerWarp * gmax || (long long)G * M > 65536) continue;
-      s->redundant = 1;
-    }
-    s->G = G;
-    s->smem = smem_doubles(s->lds, s->nsm, s->ncmax, grad) * 8;
-    return true;
-  }
-  return false;
+// Leading dimension of a block: lds / 2 odd, so that the 16-byte loads of eight
+// neighbouring columns hit all banks.
+int block_ld(int m) {
+  const int e = (m + 1) & ~1;
+  return (e >> 1) & 1 ? e : e + 2;
 }
 
-template <int RPT, bool GRAD>
+// The grid of an M x N problem; false when no grid of one block per SM holds it.
+// The cost of an iteration in clocks, as measured: about 0.17 per element of a
+// block (two passes, 16 bytes of shared memory each, at 100 B per clock) and
+// 2200 + 40 g for an exchange among g CTAs, none when a block spans the side.
+bool shape(const Context* ctx, int M, int N, Shape* best) {
+  if (ctx->sm_count > kMaxG || M > 8192) return false;  // (the general drivers refuse more rows of support)
+  double cost = 0.0;
+  bool found = false;
+  for (int gr = (M + kMaxSide - 1) / kMaxSide; gr <= std::min(M, ctx->sm_count); ++gr)
+    for (int gc = (N + kMaxSide - 1) / kMaxSide; gc <= std::min(N, ctx->sm_count / gr); ++gc) {
+      Shape s{};
+      s.gr = gr;
+      s.gc = gc;
+      s.ldm = (M + gr - 1) / gr;
+      s.ldn = (N + gc - 1) / gc;
+      const double t = 0.17 * s.ldm * s.ldn + (gr > 1 ? 2200.0 + 40.0 * gr : 0.0) + (gc > 1 ? 2200.0 + 40.0 * gc : 0.0);
+      if (found && t >= cost) continue;
+      s.lds = block_ld(s.ldm);
+      const int nrw = (s.ldm + 63) / 64;
+      s.nsm = s.ldn;
+      s.chunks = 1;
+      for (int q = 0; q < 2; ++q) {  // all columns in shared memory, else some in registers
+        const int nblk = (s.nsm + 31) / 32;
+        s.chunks = std::max(nblk > 8 ? 1 : nblk > 4 ? 2 : nblk > 2 ? 4 : nblk > 1 ? 8 : 16, q ? nrw : 1);
+        s.smem = sizeof(double) * smem_doubles(s.lds, s.ldn, s.nsm, s.chunks);
+        if (s.smem <= (size_t)ctx->smem_optin) break;
+        s.nsm = s.ldn - kRegCols * (NW / nrw);
+        s.reg = 1;
+        if (s.nsm < 1) break;
+      }
+      if (s.nsm < 1 || s.smem > (size_t)ctx->smem_optin) continue;
+      *best = s;
+      cost = t;
+      found = true;
+    }
+  return found;
+}
+
+template <bool GRAD, bool REG>
 int launch(Args& p, const Shape& s, cudaStream_t st) {
-  auto kern = resident_kernel<RPT, GRAD>;
+  auto kern = resident_kernel<GRAD, REG>;
   static size_t attr = 0;  // callers hold the context lock
   if (attr < s.smem) {
     RWIG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem));
     attr = s.smem;
   }
   void* args[] = {&p};
-  RWIG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)kern, dim3(s.G), dim3(NTT), args, s.smem, st));
+  RWIG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)kern, dim3(s.gr * s.gc), dim3(NTT), args, s.smem, st));
   return 0;
 }
 
@@ -885,10 +714,9 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   using namespace skres;
   const bool grad = grad_a != nullptr;
   Shape s;
-  if (max_iter < 1 || !(zero_tol <= 999.0) || !shape(ctx, M, N, grad, &s)) return 0;
-  const size_t L2 = (size_t)max_iter + 2;
-  const size_t hist = grad ? 8 * L2 * ((size_t)M * (s.redundant ? s.G : 1) + N) : 0;
-  if (hist > (size_t(32) << 30)) return 0;
+  if (max_iter < 1 || !(zero_tol <= 999.0) || !shape(ctx, M, N, &s)) return 0;
+  const size_t G = (size_t)s.gr * s.gc, L2 = (size_t)max_iter + 2;
+  if (grad && 8 * L2 * G * (s.ldm + s.ldn) > (size_t(32) << 30)) return 0;
   if (!ctx->resident_res) {
     void* h = nullptr;
     RWIG_CUDA_TRY(cudaHostAlloc(&h, sizeof(double) * kResWords, cudaHostAllocMapped));
@@ -896,13 +724,13 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   }
   double* dres = nullptr;
   RWIG_CUDA_TRY(cudaHostGetDevicePointer((void**)&dres, ctx->resident_res, 0));
-  const size_t npart = s.redundant ? 2 * (size_t)s.G * M : (size_t)s.G * s.G * s.R;
-  const size_t bytes = sizeof(Packet) * (npart + M + 8 * (size_t)s.G);
+  const size_t nc = 2 * (size_t)s.gr * N, nrp = 2 * (size_t)s.gc * M;
+  const size_t bytes = sizeof(Packet) * (nc + nrp + 10 * G);
   const bool fresh = (int)ctx->slots.size() <= SRS_PACKETS || ctx->slot_bytes[SRS_PACKETS] < bytes;
   Packet* pk = (Packet*)scratch(ctx, SRS_PACKETS, bytes);
   double* info = (double*)scratch(ctx, SRS_INFO, sizeof(double) * 4);
-  double* uh = grad ? (double*)scratch(ctx, SRS_UH, 8 * L2 * M * (s.redundant ? s.G : 1)) : nullptr;
-  double* vh = grad ? (double*)scratch(ctx, SRS_VH, 8 * L2 * N) : nullptr;
+  double* uh = grad ? (double*)scratch(ctx, SRS_UH, 8 * L2 * G * s.ldm) : nullptr;
+  double* vh = grad ? (double*)scratch(ctx, SRS_VH, 8 * L2 * G * s.ldn) : nullptr;
   if (!pk || !info || (grad && (!uh || !vh))) return RWIG_E_NOMEM;
   if (fresh)  // no packet of an earlier life of this memory may carry a tag to come
     RWIG_CUDA_TRY(cudaMemsetAsync(pk, 0, ctx->slot_bytes[SRS_PACKETS], st));
@@ -919,20 +747,21 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   p.info = info;
   p.M = M;
   p.N = N;
-  p.G = s.G;
-  p.R = s.R;
+  p.gr = s.gr;
+  p.gc = s.gc;
   p.lds = s.lds;
-  p.ncmax = s.ncmax;
+  p.ldm = s.ldm;
+  p.ldn = s.ldn;
   p.nsm = s.nsm;
+  p.chunks = s.chunks;
   p.vanilla = vanilla;
-  p.redundant = s.redundant;
   p.max_iter = max_iter;
   p.eps = reg;
   p.tol = zero_tol;
-  p.part = pk;
-  p.up = pk + npart;
-  p.cer = p.up + M;
-  p.fin = p.cer + 2 * s.G;
+  p.cpart = pk;
+  p.rpart = p.cpart + nc;
+  p.epart = p.rpart + nrp;
+  p.fin = p.epart + 4 * G;
   p.epoch = ++ctx->resident_epoch << 32;
   p.res = dres;
   p.err = (unsigned*)(info + 3);
@@ -942,8 +771,8 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev0, st));
   masses_kernel<<<1, NTT, 0, st>>>(a, b, M, N, info, p.err);
   int rc;
-  if (grad) rc = M <= 1024 ? launch<2, true>(p, s, st) : M <= 2048 ? launch<4, true>(p, s, st) : launch<8, true>(p, s, st);
-  else rc = M <= 1024 ? launch<2, false>(p, s, st) : M <= 2048 ? launch<4, false>(p, s, st) : launch<8, false>(p, s, st);
+  if (grad) rc = s.reg ? launch<true, true>(p, s, st) : launch<true, false>(p, s, st);
+  else rc = s.reg ? launch<false, true>(p, s, st) : launch<false, false>(p, s, st);
   if (rc) return rc;
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev1, st));
   RWIG_CUDA_TRY(cudaEventSynchronize(ctx->ev1));
