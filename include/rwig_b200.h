@@ -74,7 +74,9 @@ RWIG_API int rwig_last_report(rwig_report* out); /* report of the last call on t
  *   "log_sinkhorn.scaled": 1 (default) runs the log-Sinkhorn iterations after
  *       the first in stabilised scaling form, 0 keeps every iteration in the
  *       log domain (same results within rounding; slower);
- *   "log_sinkhorn.tau": absorption bound on |log u|, |log v| (default 100);
+ *   "log_sinkhorn.tau": absorption bound on |log u|, |log v| (default 100;
+ *       below it, and with scaled 0, a log solve never runs resident in one
+ *       launch);
  *   "log_sinkhorn.l2_hot": share of each CTA's column groups of the scaled
  *       kernel copied with an L2 evict_last hint, the rest evict_first
  *       (default 0: all evict_first; negative: no hint);
@@ -166,8 +168,7 @@ RWIG_API int rwig_sinkhorn_vanilla_dev(double* P, double* grad_a, double* u, dou
  * a: M, b: N, C: M x N.  Outputs (any may be NULL): P (M x N), grad_a (M,
  * needs withgrad), f (M), g (N; -inf off the support, as :267-270), loss.
  * grad_a is the unrolled backward Sinkhorn::_bwd_log (:379-520), zero off the
- * support; the forward of a gradient call runs every iteration in the log
- * domain, with the limits of rwig_sinkhorn_vanilla's gradient.
+ * support, with the limits of rwig_sinkhorn_vanilla's gradient.
  */
 RWIG_API int rwig_sinkhorn_log(double* P, double* grad_a, double* f, double* g, double* loss,
                       int* iter, double* err, const double* a, const double* b,

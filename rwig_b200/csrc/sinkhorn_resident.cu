@@ -36,9 +36,14 @@
 //     single 128-bit accesses: a reader polls the data itself, one trip through
 //     L2 instead of a fence, a counter and a second trip.  A tag holds the
 //     launch's number and the round, so packets need no reset;
-//   * the stopping test of an iteration runs beside the next one's column pass
-//     (whose result is thrown away when it stops).
-// The figures stand beside shape().
+//   * 15 warps iterate; the last one only forms, exchanges and judges the
+//     stopping error, two iterations behind (what was computed since is thrown
+//     away when it stops).
+// Whole solves through the C entry against the general drivers (us): 256 x 256
+// vanilla, 19 iterations 135 (430); 1777 x 1501 log, 31 iterations 328 (723);
+// with gradient 701 x 513 vanilla, 11 iterations 202 (482); 2048 x 2048 log,
+// 100 iterations 1980 (5326), 9.5 us per iteration in each direction: of about
+// 17500 clocks the two passes take 6600, the exchanges 4000-5000 each.
 #include <algorithm>
 #include <cmath>
 
@@ -49,10 +54,32 @@
 namespace rwig {
 namespace skres {
 
-constexpr int NTT = 512, NW = NTT / 32;
-constexpr int kMaxSide = 512;  // rows and columns of a block: one of each per thread
+constexpr int NW = 15, NTT = 32 * NW;  // the iterating warps
+constexpr int kThreads = NTT + 32;     // and the error warp
+constexpr int kMaxSide = NTT;          // rows and columns of a block: one of each per thread
 constexpr int kMaxG = 160;     // CTAs (five error packets per lane)
+constexpr int kPoll = 6;       // packets a thread loads at once
 constexpr int kRegCols = 4;    // REG: columns in registers per column group of the row pass
+
+// Barriers: 1 of the iterating warps; 2 and 3 hand su, suo, sd to the error
+// warp and its verdict back.
+__device__ __forceinline__ void sync() { asm volatile("bar.sync 1, 480;" ::: "memory"); }
+__device__ __forceinline__ bool sync_or(bool x) {
+  int r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, 1, 480, p;\n\tselp.s32 %0, 1, 0, "
+      "q;\n\t}"
+      : "=r"(r)
+      : "r"((int)x)
+      : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ void errors_in() { asm volatile("bar.arrive 2, 512;" ::: "memory"); }
+__device__ __forceinline__ void errors_wait() { asm volatile("bar.sync 2, 512;" ::: "memory"); }
+__device__ __forceinline__ void verdict_out() { asm volatile("bar.arrive 3, 512;" ::: "memory"); }
+__device__ __forceinline__ void verdict_wait() { asm volatile("bar.sync 3, 512;" ::: "memory"); }
+static_assert(kThreads == 512 && NTT == 480, "thread counts of the barriers");
+
 constexpr double kLo = 1e-250, kHi = 1e250;
 
 struct alignas(16) Packet {
@@ -78,7 +105,7 @@ struct Args {
   // for which it needs that peer's part in the next one first
   Packet* cpart;  // [2][gr][N] column partials
   Packet* rpart;  // [2][gc][M] row partials
-  Packet* epart;  // [2][2][G]  error shares: rows, columns
+  Packet* epart;  // [4][G][2]  error shares: rows, columns (four: read one iteration after they are sent)
   Packet* fin;    // [G][6]
   unsigned long long epoch;  // launch number << 32
   double* res;               // host-mapped results (kRes*)
@@ -180,7 +207,7 @@ __host__ __device__ constexpr size_t smem_doubles(int lds, int ldn, int nsm, int
 // REG: the last kRegCols columns per column group of the row pass are held in
 // registers (nsm of the block's columns in shared memory).
 template <bool GRAD, bool REG>
-__global__ void __launch_bounds__(NTT, 1) resident_kernel(Args p) {
+__global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
   extern __shared__ __align__(128) double sm[];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, cta = blockIdx.x;
   const int M = p.M, N = p.N, gr = p.gr, gc = p.gc, G = gr * gc, lds = p.lds, ldn = p.ldn;
@@ -217,33 +244,78 @@ __global__ void __launch_bounds__(NTT, 1) resident_kernel(Args p) {
   if (tid < mr) sa[tid] = a_i;
   if (tid < nr) sb[tid] = b_j;
   for (int i = mr + tid; i < lds; i += NTT) su[i] = 0.0;
+  for (int c = tid; c < ns; c += NTT)
+    for (int i = mr; i < lds; ++i) K[(size_t)c * lds + i] = 0.0;
   bool bad = false, ok = true;
   // tags: the launch and the number of the exchange, counted for each kind apart
-  unsigned long long ct = p.epoch, rt = p.epoch, et = p.epoch;
+  unsigned long long ct = p.epoch, rt = p.epoch;
 
-  // K = exp(-C/eps) of the block, elements spread over the threads
-  auto build = [&]() {
-    auto entry = [&](double c) {
-      const double x = exp(-c / eps);
-      if (!p.vanilla && !(x >= 2.2250738585072014e-308 && x <= 1.79e308)) bad = true;
-      return x;
-    };
-    const int el = ns * mr;
-#pragma unroll 4
-    for (int e = tid; e < el; e += NTT) {
-      const int c = e / mr, i = e - c * mr;
-      K[(size_t)c * lds + i] = entry(p.C[(size_t)(n0 + c) * M + m0 + i]);
+  // fn(C_ij, i, j) for the block's elements in shared memory, spread over the
+  // threads, four loads at a time
+  auto each = [&](auto fn) {
+    const int dc = NTT / mr, di = NTT - dc * mr;
+    int c = tid / mr, i = tid - c * mr;
+    const double* const Cb = p.C + (size_t)n0 * M + m0;
+    while (c < ns) {
+      double x[4];
+      int cc[4], ii[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        cc[k] = c;
+        ii[k] = i;
+        x[k] = c < ns ? Cb[(size_t)c * M + i] : 0.0;
+        c += dc;
+        i += di;
+        if (i >= mr) {
+          i -= mr;
+          ++c;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (cc[k] < ns) fn(x[k], ii[k], cc[k]);
     }
-    for (int c = tid; c < ns; c += NTT)
-      for (int i = mr; i < lds; ++i) K[(size_t)c * lds + i] = 0.0;
+  };
+  // What stands in the block's place: K = exp(-C/eps) (kind 0), the plan P (1),
+  // or pb = (C + eps log P) o P (2); su, sd hold f, g for the latter two.
+  double l1 = 0.0, l2 = 0.0;
+  bool zero_plan = false;
+  auto fill = [&](int kind) {
+    auto entry = [&](double c, int i, int j) {
+      if (kind == 0) {
+        const double x = exp(-c / eps);
+        if (!p.vanilla && !(x >= 2.2250738585072014e-308 && x <= 1.79e308)) bad = true;
+        return x;
+      }
+      if (sa[i] == 0.0 || sb[j] == 0.0) return 0.0;
+      const double x = -((c - su[i]) - sd[j]) * inv_eps;
+      const double pv = exp(x);
+      // log P: x itself, from which the logarithm of the rounded P differs by
+      // less than one unit of the last place of 1; minus infinity where P underflowed
+      const double lp = pv > 0.0 ? x : -INFINITY;
+      if (kind == 2) return (c + eps * lp) * pv;
+      l1 += c * pv;
+      l2 += pv * (lp - 1.0);
+      zero_plan |= !(pv > 0.0);
+      return pv;
+    };
+    double* const Pb = kind == 1 && p.P ? p.P + (size_t)n0 * M + m0 : nullptr;
+    each([&](double cij, int i, int c) {
+      const double x = entry(cij, i, c);
+      K[(size_t)c * lds + i] = x;
+      if (Pb) Pb[(size_t)c * M + i] = x;
+    });
     if constexpr (REG) {
+      const double* const Cb = p.C + (size_t)n0 * M + m0;
 #pragma unroll
       for (int q = 0; q < kRegCols; ++q) {
         const int c = ns + grp * kRegCols + q;
-        const bool in = row_ok && c < nr;
-        const double* Cc = p.C + (size_t)(n0 + c) * M + m0 + r0;
-        kr[q].x = in ? entry(Cc[0]) : 0.0;
-        kr[q].y = in && r0 + 1 < mr ? entry(Cc[1]) : 0.0;
+        const size_t at = (size_t)c * M + r0;
+        const bool in = row_ok && c < nr, in1 = in && r0 + 1 < mr;
+        kr[q].x = in ? entry(Cb[at], r0, c) : 0.0;
+        kr[q].y = in1 ? entry(Cb[at + 1], r0 + 1, c) : 0.0;
+        if (Pb && in) Pb[at] = kr[q].x;
+        if (Pb && in1) Pb[at + 1] = kr[q].y;
       }
     }
   };
@@ -272,46 +344,47 @@ __global__ void __launch_bounds__(NTT, 1) resident_kernel(Args p) {
       rowp[grp * mr + r0] = x;
       if (r0 + 1 < mr) rowp[grp * mr + r0 + 1] = y;
     }
-    __syncthreads();
+    sync();
+  };
+  // Sends this thread's partial t (mine: it has one) as sender `me` of n and adds
+  // all n in order.  Whole warps; packets of sender e at base + e ld + tid.
+  auto exchange = [&](Packet* base, int ld, int n, int me, bool mine, double t, unsigned long long tag) {
+    Packet* const q = base + tid;
+    if (mine) put(q + (size_t)me * ld, t, tag);
+    t = 0.0;
+    if (mine)
+      for (int k = 0; k < n && ok; k += kPoll) {
+        double x[kPoll];
+        ok = poll<kPoll>(min(kPoll, n - k), [&](int e) { return q + (size_t)(k + e) * ld; }, tag, x, p.err);
+#pragma unroll
+        for (int e = 0; e < kPoll; ++e) t += x[e];
+      }
+    return t;
   };
   // The rows' totals over the block row (thread tid < mr: row m0 + tid): this
-  // CTA's partial (`extra` minus it, when given) sent and all gc added in order.
-  auto row_total = [&](const double* extra) {
+  // CTA's partial (rest: `extra` minus it) sent and all gc added in order.
+  auto row_total = [&](bool rest, double extra) {
     double t = 0.0;
     const unsigned long long tag = ++rt;
     if (tid < mr) {
       for (int q = 0; q < ngrp; ++q) t += rowp[q * mr + tid];
-      if (extra) t = *extra - t;
-      if (gc > 1) {
-        Packet* base = p.rpart + (tag & 1) * (size_t)gc * M + m0 + tid;
-        put(base + (size_t)ci * M, t, tag);
-        t = 0.0;
-        for (int k = 0; k < gc && ok; k += 12) {
-          double x[12];
-          ok = poll<12>(min(12, gc - k), [&](int e) { return base + (size_t)(k + e) * M; }, tag, x, p.err);
-#pragma unroll
-          for (int e = 0; e < 12; ++e) t += x[e];
-        }
-      }
+      if (rest) t = extra - t;
     }
+    if (gc > 1 && 32 * w < mr) t = exchange(p.rpart + (tag & 1) * (size_t)gc * M + m0, M, gc, ci, tid < mr, t, tag);
     return t;
   };
   // Column pass: partial sums over the block's rows of K^T su -> colp[chunk][ldn];
   // returns the chunks (register columns: nrw).
   const int nblk = (p.nsm + 31) >> 5;  // (the same in every CTA: it sizes colp)
-  const int lg = nblk > 8 ? 4 : nblk > 4 ? 3 : nblk > 2 ? 2 : nblk > 1 ? 1 : 0;
-  const int nrc = NW >> lg;
+  const int nrc = NW / nblk;           // row chunks: nblk x nrc warps
+  const int blk = w / nrc, chunk = w - blk * nrc;
   const int pairs = (mr + 1) >> 1;
-  const int p0 = (w & (nrc - 1)) * pairs >> (4 - lg), p1 = ((w & (nrc - 1)) + 1) * pairs >> (4 - lg);
+  const int p0 = chunk * pairs / nrc, p1 = (chunk + 1) * pairs / nrc;
   auto col_pass = [&]() {
-    for (int blk = w >> (4 - lg); blk < nblk; blk += 1 << lg) {
-      const int c0 = 32 * blk, nq = (min(32, ns - c0) + 7) >> 3;
-      double* out = colp + (w & (nrc - 1)) * ldn;
-      if (nq == 4) sum_block<4>(K, lds, ns, c0, p0, p1, su, out);
-      else if (nq == 3) sum_block<3>(K, lds, ns, c0, p0, p1, su, out);
-      else if (nq == 2) sum_block<2>(K, lds, ns, c0, p0, p1, su, out);
-      else sum_block<1>(K, lds, ns, c0, p0, p1, su, out);
-    }
+    const int c0 = 32 * blk;
+    double* out = colp + chunk * ldn;
+    if (c0 + 16 < ns) sum_block<4>(K, lds, ns, c0, p0, p1, su, out);
+    else if (c0 < ns) sum_block<2>(K, lds, ns, c0, p0, p1, su, out);
     if constexpr (REG) {
       const double u0 = row_ok ? su[r0] : 0.0, u1 = row_ok ? su[r0 + 1] : 0.0;
 #pragma unroll
@@ -321,7 +394,7 @@ __global__ void __launch_bounds__(NTT, 1) resident_kernel(Args p) {
         if (lane == 0 && in_pass && c < nr) colp[rw * ldn + c] = x;
       }
     }
-    __syncthreads();
+    sync();
   };
   // The columns' totals over the block column (thread tid < nr: column n0 + tid).
   auto col_total = [&]() {
@@ -330,69 +403,30 @@ __global__ void __launch_bounds__(NTT, 1) resident_kernel(Args p) {
     if (tid < nr) {
       const int n = REG && tid >= ns ? nrw : nrc;
       for (int q = 0; q < n; ++q) t += colp[q * ldn + tid];
-      if (gr > 1) {
-        Packet* base = p.cpart + (tag & 1) * (size_t)gr * N + n0 + tid;
-        put(base + (size_t)ri * N, t, tag);
-        t = 0.0;
-        for (int k = 0; k < gr && ok; k += 12) {
-          double x[12];
-          ok = poll<12>(min(12, gr - k), [&](int e) { return base + (size_t)(k + e) * N; }, tag, x, p.err);
-#pragma unroll
-          for (int e = 0; e < 12; ++e) t += x[e];
-        }
-      }
     }
+    if (gr > 1 && 32 * w < nr) t = exchange(p.cpart + (tag & 1) * (size_t)gr * N + n0, N, gr, ri, tid < nr, t, tag);
     return t;
   };
   auto in_range = [](double x) { return x >= kLo && x <= kHi; };
-  double* const uh = GRAD ? p.uh + (size_t)cta * (p.max_iter + 2) * p.ldm : nullptr;
-  double* const vh = GRAD ? p.vh + (size_t)cta * (p.max_iter + 2) * ldn : nullptr;
-  // Sum over CTAs of error share q of exchange et, by one warp.
-  auto error_at = [&](int q) { return p.epart + ((et & 1) * 2 + q) * G; };
-  auto error_sum = [&](int q) {
-    double x[kMaxG / 32], t = 0.0;
-    const Packet* base = error_at(q);
-    const unsigned long long tag = et;
-    ok = poll<kMaxG / 32>((G - lane + 31) >> 5, [&](int k) { return base + lane + 32 * k; }, tag, x, p.err) && ok;
-#pragma unroll
-    for (int k = 0; k < kMaxG / 32; ++k) t += x[k];
-    return warp_sum(t);
-  };
+  double* const uh = GRAD ? p.uh + (size_t)cta * (p.max_iter + 4) * p.ldm : nullptr;
+  double* const vh = GRAD ? p.vh + (size_t)cta * (p.max_iter + 4) * ldn : nullptr;
+  // Packets of exchange e: each CTA's shares of the row and the column error.
+  auto error_at = [&](unsigned long long e) { return p.epart + (e & 3) * 2 * G; };
 
-  // ---------------------------------------------------------------- forward
-  build();
-  if (tid < nr) {
-    sv[tid] = b_j != 0.0 ? 1.0 : 0.0;  // K 1 over the support
-    sd[tid] = 0.0;
-  }
-  bad = __syncthreads_or(bad);
-  // each CTA's share of the error: rows and columns of its block's row and column
-  const int ea = ci * mr / gc, eb = (ci + 1) * mr / gc, ec0 = ri * nr / gr, ec1 = (ri + 1) * nr / gr;
-  int iter = 0;
-  double err = 1000.0, u = 1.0, v = 0.0, vo = 0.0;
-  row_pass();
-  u = row_total(nullptr);
-  // iteration k = iter + 1: u_k from the totals, v_k, totals of K v_k
-  while (true) {
-    const double uo = iter > 0 ? su[tid < mr ? tid : 0] : 0.0;
-    u = a_i == 0.0 ? 0.0 : in_range(u) ? a_i / u : INFINITY;  // (an infinite u fails the range check below)
-    if (tid < mr) {
-      suo[tid] = uo;
-      su[tid] = u;
-      if (GRAD) uh[(size_t)(iter + 1) * p.ldm + tid] = u;
-    }
-    if (__syncthreads_or(!ok)) {
-      ok = false;
-      break;
-    }
-    ++et;
-    if (w == NW - 1) {  // this CTA's share of the last iteration's error (of iteration 0: the range checks)
-      double e = bad ? INFINITY : 0.0, ec = 0.0;
+  // ---------------------------------------------------------------- error warp
+  if (w == NW) {
+    // this CTA's share: rows and columns of its block's row and column
+    const int ea = ci * mr / gc, eb = (ci + 1) * mr / gc, ec0 = ri * nr / gr, ec1 = (ri + 1) * nr / gr;
+    for (int k = 1;; ++k) {  // loop k: u_k is in su, u_{k-1} in suo, the terms of v_{k-1} in sd
+      errors_wait();
+      if (es[2] != 0.0) return;
+      const unsigned long long now = p.epoch + k, last = now - 1;
+      double e = 0.0, ec = 0.0;
       for (int i = ea + lane; i < eb; i += 32) {
         const double a = sa[i], x = su[i];
         if (a == 0.0) continue;
         if (!in_range(x)) e = INFINITY;
-        else if (iter > 0) {
+        else if (k > 1) {
           const double q = suo[i] / x;  // u_i (K v)_i / a_i
           const double d = p.vanilla ? a * (q - 1.0) : log(q);
           e = fma(d, d, e);
@@ -401,231 +435,242 @@ __global__ void __launch_bounds__(NTT, 1) resident_kernel(Args p) {
       for (int c = ec0 + lane; c < ec1; c += 32) ec += sd[c];
       e = warp_sum(e);
       ec = warp_sum(ec);
-      if (lane < 2) put(error_at(lane) + cta, lane ? ec : e, et);
-    }
-    col_pass();
-    const double s = col_total();
-    if (w == NW - 1) {
-      const double e0 = error_sum(0), e1 = error_sum(1);
-      if (lane == 0) {
-        const double e = sqrt(e0) + sqrt(e1);
-        es[0] = e;
-        es[1] = !(e0 + e1 <= 1e300) ? 2.0 : iter > 0 && !(iter < p.max_iter && e >= p.tol) ? 1.0 : 0.0;
+      if (k == 1 && es[3] != 0.0) e = INFINITY;  // K has subnormal entries
+      if (lane < 2) put(error_at(now) + 2 * cta + lane, lane ? ec : e, now);
+      double verdict = 0.0, er = 0.0;
+      if (k > 1) {  // iteration k - 2 (of iteration 0: the range checks)
+        constexpr int NP = 2 * kMaxG / 32;
+        double x[NP], t[2] = {0.0, 0.0};
+        const int n = (G - lane + 31) >> 5;
+        const bool ok = poll<NP>(2 * n, [&](int q) { return error_at(last) + 2 * (lane + 32 * (q >> 1)) + (q & 1); }, last, x, p.err);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) t[q & 1] += x[q];
+        const double e0 = warp_sum(t[0]), e1 = warp_sum(t[1]);
+        er = sqrt(e0) + sqrt(e1);
+        verdict = __any_sync(0xffffffffu, !ok) ? 3.0 : !(e0 + e1 <= 1e300) ? 2.0
+                  : k > 2 && !(k - 2 < p.max_iter && er >= p.tol) ? 1.0 : 0.0;
       }
+      if (lane == 0) {
+        es[0] = er;
+        es[1] = verdict;
+      }
+      __syncwarp();
+      verdict_out();
+      if (verdict != 0.0) return;
     }
-    vo = v;
-    v = b_j / s;
-    if (b_j == 0.0) v = 0.0;
-    __syncthreads();  // (the row pass and the error share have read sv and sd)
-    if (es[1] != 0.0) break;
-    if (tid < nr) {
-      sv[tid] = v;
-      const double d = p.vanilla ? fma(v, s, -b_j) : fma(v, s, -b_j) * rb_j;  // log(v s / b) to first order
-      sd[tid] = b_j == 0.0 ? 0.0 : in_range(s) && in_range(v) ? d * d : INFINITY;
-      if (GRAD) vh[(size_t)(iter + 1) * ldn + tid] = v;
+  }
+
+  // ---------------------------------------------------------------- iterating warps
+  // One loop runs every stage of the solve, so that the passes and exchanges
+  // are in the code once (inlined per stage, the loop outgrew the instruction
+  // cache: 16000 clocks for an exchange of the backward steps).
+  enum { kInit, kForward, kMargins, kMargins2, kBackward0, kBackward };
+  int stage = kInit, kind = 0;
+  int k = 0, l = 0, iter = 0;
+  double err = 0.0;
+  double u = 0.0, u1 = 0.0, u2 = 0.0, v = 0.0, v1 = 0.0, v2 = 0.0;  // of this and the last two iterations
+  double s = 0.0, t = 0.0;      // column and row totals
+  double fi = 0.0, ex = 0.0, ga = 0.0, ul = 0.0, vl = 0.0;
+  unsigned long long et = 0, t_b = 0;
+  while (true) {
+    if (kind >= 0) {  // (synchronised before)
+      fill(kind);
+      const bool any = sync_or(bad);
+      if (stage == kInit) {
+        if (tid < nr) {
+          sv[tid] = b_j != 0.0 ? 1.0 : 0.0;  // K 1 over the support
+          sd[tid] = 0.0;
+        }
+        if (tid == 0) {
+          es[1] = es[2] = 0.0;
+          es[3] = any ? 1.0 : 0.0;
+        }
+      } else if (stage == kBackward0) {
+        if (tid < nr) sv[tid] = b_j != 0.0 ? s * v * rb_j : 0.0;
+      } else {
+        if (tid < mr) su[tid] = 1.0;
+        if (tid < nr) sv[tid] = 1.0;
+      }
+      kind = -1;
+      sync();
     }
-    ++iter;
-    if (__syncthreads_or(!ok)) {
+    if (stage != kInit && stage != kBackward0) {
+      col_pass();
+      s = col_total();
+    }
+    if (stage == kForward) {
+      v2 = v1;
+      v1 = v;
+      v = b_j == 0.0 ? 0.0 : b_j / s;
+      verdict_wait();  // (and everyone is done with sv and sd)
+      if (es[1] != 0.0) {
+        // iteration k - 2 is the last: its potentials, then the plan
+        iter = k - 2;
+        err = es[0];
+        u = u2;
+        v = v2;
+        fi = eps * log(u);
+        const double gj = eps * log(v);
+        if (es[1] != 1.0) break;
+        sync();
+        if (tid < mr) {
+          su[tid] = fi;
+          if (ci == 0 && p.f) p.f[m0 + tid] = p.vanilla ? u : fi;
+        }
+        if (tid < nr) {
+          sd[tid] = gj;
+          if (ri == 0 && p.g) p.g[n0 + tid] = p.vanilla ? v : gj;
+        }
+        et = p.epoch + k + 1;
+        stage = kMargins;
+        kind = 1;
+        sync();
+        continue;
+      }
+      if (tid < nr) {
+        sv[tid] = v;
+        const double d = p.vanilla ? fma(v, s, -b_j) : fma(v, s, -b_j) * rb_j;  // log(v s / b) to first order
+        sd[tid] = b_j == 0.0 ? 0.0 : in_range(s) && in_range(v) ? d * d : INFINITY;
+        if (GRAD) vh[(size_t)k * ldn + tid] = v;
+      }
+    } else if (GRAD && stage == kBackward) {
+      if (tid < nr) sv[tid] = s * (vl * vl) * rb_j;
+    }
+    if (sync_or(!ok)) {
       ok = false;
       break;
     }
     row_pass();
-    u = row_total(nullptr);
-  }
-  ok = !__syncthreads_or(!ok);
-  if (!ok || es[1] == 2.0) {
-    if (cta == 0 && tid == 0) {
-      p.res[kResKerr] = ok ? 0.0 : 1.0;
-      p.res[kResStatus] = kResUnsafe;
-    }
-    return;
-  }
-  err = es[0];
-  u = tid < mr ? suo[tid] : 0.0;  // the stopped iteration's scalings
-  v = vo;
+    t = row_total(GRAD && stage == kBackward0, ex);
 
-  // ---------------------------------------------------------------- plan, loss, marginals
-  const double fi = eps * log(u), gj = eps * log(v);
-  __syncthreads();
-  if (tid < mr) {
-    su[tid] = fi;
-    if (ci == 0 && p.f) p.f[m0 + tid] = p.vanilla ? u : fi;
-  }
-  if (tid < nr) {
-    sd[tid] = gj;
-    if (ri == 0 && p.g) p.g[n0 + tid] = p.vanilla ? v : gj;
-  }
-  __syncthreads();
-  double l1 = 0.0, l2 = 0.0;
-  bool zero_plan = false;
-  // P (pass 0) or pb = (C + eps log P) o P (pass 1) in K's place
-  auto plan = [&](int pass) {
-    auto entry = [&](double c, int i, int j) {
-      if (sa[i] == 0.0 || sb[j] == 0.0) return 0.0;
-      const double x = -((c - su[i]) - sd[j]) * inv_eps;
-      const double pv = exp(x);
-      // log P: x itself, which exp's rounding moves by less than one unit of
-      // the last place of 1; minus infinity where P underflowed
-      const double lp = pv > 0.0 ? x : -INFINITY;
-      if (pass == 0) {
-        l1 += c * pv;
-        l2 += pv * (lp - 1.0);
-        zero_plan |= !(pv > 0.0);
+    if (stage <= kForward) {  // iteration k: u_k from the totals of K v_{k-1}
+      stage = kForward;
+      ++k;
+      u2 = u1;
+      u1 = u;
+      u = a_i == 0.0 ? 0.0 : in_range(t) ? a_i / t : INFINITY;  // (an infinite u fails the error warp's check)
+      if (tid < mr) {
+        suo[tid] = u1;
+        su[tid] = u;
+        if (GRAD) uh[(size_t)k * p.ldm + tid] = u;
       }
-      return pass == 0 ? pv : (c + eps * lp) * pv;
-    };
-    const int el = ns * mr;
-#pragma unroll 2
-    for (int e = tid; e < el; e += NTT) {
-      const int c = e / mr, i = e - c * mr;
-      const size_t at = (size_t)(n0 + c) * M + m0 + i;
-      const double x = entry(p.C[at], i, c);
-      K[(size_t)c * lds + i] = x;
-      if (pass == 0 && p.P) p.P[at] = x;
-    }
-    if constexpr (REG) {
-#pragma unroll
-      for (int q = 0; q < kRegCols; ++q) {
-        const int c = ns + grp * kRegCols + q;
-        if (!(row_ok && c < nr)) continue;
-        const size_t at = (size_t)(n0 + c) * M + m0 + r0;
-        kr[q].x = entry(p.C[at], r0, c);
-        if (pass == 0 && p.P) p.P[at] = kr[q].x;
-        if (r0 + 1 < mr) {
-          kr[q].y = entry(p.C[at + 1], r0 + 1, c);
-          if (pass == 0 && p.P) p.P[at + 1] = kr[q].y;
-        }
-      }
-    }
-    __syncthreads();
-  };
-  // row and column sums of what stands in K's place (su, sv: ones)
-  auto margins = [&](double& row, double& col) {
-    if (tid < mr) su[tid] = 1.0;
-    if (tid < nr) sv[tid] = 1.0;
-    __syncthreads();
-    col_pass();
-    col = col_total();
-    row_pass();
-    row = row_total(nullptr);
-    __syncthreads();
-  };
-  double row = 0.0, col = 0.0;
-  plan(0);
-  margins(row, col);
-  {
-    const bool ra = ci == 0 && tid < mr && a_i != 0.0, cb = ri == 0 && tid < nr && b_j != 0.0;
-    const double dr = ra ? row - a_i : 0.0, dc = cb ? col - b_j : 0.0;
-    const double t6[6] = {l1, l2, fabs(dc), dc * dc, fabs(dr), dr * dr};
-#pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      const double x = warp_sum(t6[t]);
-      if (lane == 0) rowp[t * NW + w] = x;
-    }
-    const bool zp = __syncthreads_or(zero_plan);
-    if (tid < 6) {
-      double t = 0.0;
-      for (int q = 0; q < NW; ++q) t += rowp[tid * NW + q];
-      put(p.fin + cta * 6 + tid, t, p.epoch);
-    }
-    ++et;
-    if (GRAD && tid == 0) put(error_at(0) + cta, zp ? INFINITY : 0.0, et);
-  }
-  if (cta == 0) {
-    if (w < 6) {
-      double x[kMaxG / 32], t = 0.0;
-      ok = poll<kMaxG / 32>((G - lane + 31) >> 5, [&](int k) { return p.fin + (lane + 32 * k) * 6 + w; }, p.epoch, x, p.err) && ok;
-#pragma unroll
-      for (int k = 0; k < kMaxG / 32; ++k) t += x[k];
-      t = warp_sum(t);
-      if (lane == 0) es[2 + w] = t;
-    }
-    ok = !__syncthreads_or(!ok || *(volatile unsigned*)p.err != 0u);
-    if (tid == 0) {
-      p.res[kResIter] = iter;
-      p.res[kResErr] = err;
-      p.res[kResLoss] = es[2] + eps * es[3];
-      p.res[kResL1Row] = es[6];
-      p.res[kResL1Col] = es[4];
-      p.res[kResL2Row] = sqrt(es[7]);
-      p.res[kResL2Col] = sqrt(es[5]);
-      p.res[kResSupM] = p.info[0];
-      p.res[kResSupN] = p.info[1];
-      p.res[kResGradNs] = 0.0;
-      p.res[kResKerr] = ok ? 0.0 : 1.0;
-      if (!GRAD || !ok) p.res[kResStatus] = ok ? kResFinished : kResUnsafe;
-    }
-  }
-  if constexpr (GRAD) {
-    // -------------------------------------------------------------- backward
-    const unsigned long long t_b = globaltimer_ns();
-    // a plan entry that underflowed: the reference's sums turn NaN or infinite
-    // there, which the general path reproduces
-    if (w == 0) {
-      const double t = error_sum(0);
-      if (lane == 0) es[1] = t;
-    }
-    ok = !__syncthreads_or(!ok);
-    if (!ok || !(es[1] <= 1e300)) {
-      if (cta == 0 && tid == 0) {
-        p.res[kResKerr] = ok ? 0.0 : 1.0;
-        p.res[kResStatus] = kResUnsafe;
-      }
-      return;
-    }
-    if (tid < mr) su[tid] = fi;
-    __syncthreads();
-    plan(1);
-    margins(row, col);
-    build();
-    if (tid < nr) sv[tid] = b_j != 0.0 ? col * v * rb_j : 0.0;
-    // (pb 1) / u: the whole row total here, so one CTA of the block row brings it in
-    const double ex = ci == 0 && a_i != 0.0 ? row / u : 0.0;
-    __syncthreads();
-    row_pass();
-    double t = row_total(&ex), ga = 0.0;
-    for (int l = iter;; --l) {
-      const double ul = tid < mr && a_i != 0.0 ? uh[(size_t)l * p.ldm + tid] : 0.0;  // written by this thread
-      const double q = a_i != 0.0 ? t * ul / a_i : 0.0;
-      ga += q;
-      if (l == 1) break;
-      const double vl = tid < nr ? vh[(size_t)(l - 1) * ldn + tid] : 0.0;
-      if (tid < mr) su[tid] = q * ul;
-      if (__syncthreads_or(!ok)) {
+      if (sync_or(!ok)) {
         ok = false;
         break;
       }
-      col_pass();
-      const double s = col_total();
-      if (tid < nr) sv[tid] = s * (vl * vl) * rb_j;
-      __syncthreads();
-      row_pass();
-      t = row_total(nullptr);
+      errors_in();
+    } else if (stage == kMargins) {
+      // loss and marginals to CTA 0
+      const bool ra = ci == 0 && tid < mr && a_i != 0.0, cb = ri == 0 && tid < nr && b_j != 0.0;
+      const double dr = ra ? t - a_i : 0.0, dc = cb ? s - b_j : 0.0;
+      const double t6[6] = {l1, l2, fabs(dc), dc * dc, fabs(dr), dr * dr};
+      sync();
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        const double x = warp_sum(t6[q]);
+        if (lane == 0) rowp[q * NW + w] = x;
+      }
+      const bool zp = sync_or(zero_plan);
+      if (tid < 6) {
+        double x = 0.0;
+        for (int q = 0; q < NW; ++q) x += rowp[tid * NW + q];
+        put(p.fin + cta * 6 + tid, x, p.epoch);
+      }
+      if (GRAD && tid == 0) put(error_at(et) + 2 * cta, zp ? INFINITY : 0.0, et);
+      if (cta == 0) {
+        if (w < 6) {
+          double x[kMaxG / 32], y = 0.0;
+          ok = poll<kMaxG / 32>((G - lane + 31) >> 5, [&](int q) { return p.fin + (lane + 32 * q) * 6 + w; }, p.epoch, x, p.err) && ok;
+#pragma unroll
+          for (int q = 0; q < kMaxG / 32; ++q) y += x[q];
+          y = warp_sum(y);
+          if (lane == 0) es[2 + w] = y;
+        }
+        sync();
+        if (tid == 0) {
+          p.res[kResIter] = iter;
+          p.res[kResErr] = err;
+          p.res[kResLoss] = es[2] + eps * es[3];
+          p.res[kResL1Row] = es[6];
+          p.res[kResL1Col] = es[4];
+          p.res[kResL2Row] = sqrt(es[7]);
+          p.res[kResL2Col] = sqrt(es[5]);
+          p.res[kResSupM] = p.info[0];
+          p.res[kResSupN] = p.info[1];
+          p.res[kResGradNs] = 0.0;
+        }
+      }
+      if (!GRAD) break;
+      t_b = globaltimer_ns();
+      // a plan entry that underflowed: the reference's sums turn NaN or infinite
+      // there, which the general path reproduces
+      if (w == 0) {
+        double x[kMaxG / 32], y = 0.0;
+        ok = poll<kMaxG / 32>((G - lane + 31) >> 5, [&](int q) { return error_at(et) + 2 * (lane + 32 * q); }, et, x, p.err) && ok;
+#pragma unroll
+        for (int q = 0; q < kMaxG / 32; ++q) y += x[q];
+        y = warp_sum(y);
+        if (lane == 0) es[1] = y <= 1e300 ? 1.0 : 2.0;
+      }
+      if (tid < mr) su[tid] = fi;
+      stage = kMargins2;
+      kind = 2;
+      if (sync_or(!ok)) {
+        ok = false;
+        break;
+      }
+      if (es[1] != 1.0) break;
+    } else if (stage == kMargins2) {
+      // (pb 1) / u: the whole row total, so one CTA of the block row brings it in
+      ex = ci == 0 && a_i != 0.0 ? t / u : 0.0;
+      stage = kBackward0;
+      kind = 0;
+      l = iter;
+      ul = u;
+      sync();
+    } else {  // step l: x = ubar u_l^2 / a, grad += ubar u_l / a
+      const double q = a_i != 0.0 ? t * ul / a_i : 0.0;
+      ga += q;
+      --l;
+      if (l == 0) break;
+      if (tid < mr) su[tid] = q * ul;
+      ul = tid < mr && a_i != 0.0 ? uh[(size_t)l * p.ldm + tid] : 0.0;  // (written by this thread)
+      vl = tid < nr ? vh[(size_t)l * ldn + tid] : 0.0;
+      stage = kBackward;
+      if (sync_or(!ok)) {
+        ok = false;
+        break;
+      }
     }
-    if (ci == 0 && tid < mr) p.grad[m0 + tid] = ga;
-    ok = !__syncthreads_or(!ok || *(volatile unsigned*)p.err != 0u);
-    if (cta == 0 && tid == 0) {
-      p.res[kResGradNs] = (double)(globaltimer_ns() - t_b);
-      p.res[kResKerr] = ok ? 0.0 : 1.0;
-      p.res[kResStatus] = ok ? kResFinished : kResUnsafe;
-    }
+  }
+  ok = !sync_or(!ok || *(volatile unsigned*)p.err != 0u);
+  if (es[1] == 0.0) {  // left before a verdict: let the error warp go
+    if (tid == 0) es[2] = 1.0;
+    errors_in();
+  }
+  const bool done = ok && es[1] == 1.0;
+  if (GRAD && done && ci == 0 && tid < mr) p.grad[m0 + tid] = ga;
+  if (cta == 0 && tid == 0) {
+    if (GRAD && done) p.res[kResGradNs] = (double)(globaltimer_ns() - t_b);
+    p.res[kResKerr] = ok && es[1] != 3.0 ? 0.0 : 1.0;
+    p.res[kResStatus] = done ? kResFinished : kResUnsafe;
   }
 }
 
 // Support sizes (non-zero masses) and whether a mass is one the scaling form
 // does not take (negative or not finite) or a side has none; clears *err.
-__global__ void __launch_bounds__(NTT) masses_kernel(const double* a, const double* b, int M, int N, double* info,
+__global__ void __launch_bounds__(kThreads) masses_kernel(const double* a, const double* b, int M, int N, double* info,
                                                      unsigned* err) {
   __shared__ int cnt[2];
   if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
   __syncthreads();
   int ca = 0, cbn = 0, bad = 0;
-  for (int i = threadIdx.x; i < M; i += NTT) {
+  for (int i = threadIdx.x; i < M; i += kThreads) {
     const double x = a[i];
     ca += x != 0.0;
     bad |= !(x >= 0.0 && x <= 1e300);
   }
-  for (int j = threadIdx.x; j < N; j += NTT) {
+  for (int j = threadIdx.x; j < N; j += kThreads) {
     const double x = b[j];
     cbn += x != 0.0;
     bad |= !(x >= 0.0 && x <= 1e300);
@@ -657,6 +702,8 @@ int block_ld(int m) {
 // The cost of an iteration in clocks, as measured: about 0.17 per element of a
 // block (two passes, 16 bytes of shared memory each, at 100 B per clock) and
 // 2200 + 40 g for an exchange among g CTAs, none when a block spans the side.
+// A problem that fits on the chip always goes here: from 120 x 95 (one CTA: 237
+// us a call against 571) to 2048^2 (1980 against 5326) the general drivers lost.
 bool shape(const Context* ctx, int M, int N, Shape* best) {
   if (ctx->sm_count > kMaxG || M > 8192) return false;  // (the general drivers refuse more rows of support)
   double cost = 0.0;
@@ -675,8 +722,7 @@ bool shape(const Context* ctx, int M, int N, Shape* best) {
       s.nsm = s.ldn;
       s.chunks = 1;
       for (int q = 0; q < 2; ++q) {  // all columns in shared memory, else some in registers
-        const int nblk = (s.nsm + 31) / 32;
-        s.chunks = std::max(nblk > 8 ? 1 : nblk > 4 ? 2 : nblk > 2 ? 4 : nblk > 1 ? 8 : 16, q ? nrw : 1);
+        s.chunks = std::max(NW / ((s.nsm + 31) / 32), q ? nrw : 1);
         s.smem = sizeof(double) * smem_doubles(s.lds, s.ldn, s.nsm, s.chunks);
         if (s.smem <= (size_t)ctx->smem_optin) break;
         s.nsm = s.ldn - kRegCols * (NW / nrw);
@@ -700,7 +746,7 @@ int launch(Args& p, const Shape& s, cudaStream_t st) {
     attr = s.smem;
   }
   void* args[] = {&p};
-  RWIG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)kern, dim3(s.gr * s.gc), dim3(NTT), args, s.smem, st));
+  RWIG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)kern, dim3(s.gr * s.gc), dim3(kThreads), args, s.smem, st));
   return 0;
 }
 
@@ -715,8 +761,11 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   const bool grad = grad_a != nullptr;
   Shape s;
   if (max_iter < 1 || !(zero_tol <= 999.0) || !shape(ctx, M, N, &s)) return 0;
-  const size_t G = (size_t)s.gr * s.gc, L2 = (size_t)max_iter + 2;
-  if (grad && 8 * L2 * G * (s.ldm + s.ldn) > (size_t(32) << 30)) return 0;
+  const size_t G = (size_t)s.gr * s.gc, L2 = (size_t)max_iter + 4;
+  // each CTA keeps its own scalings of every iteration, which takes gr + gc
+  // times the general drivers' history: at most 4 GB of it (2048^2: max_iter
+  // 10000), and the general drivers when it cannot be had
+  if (grad && 8 * L2 * G * (s.ldm + s.ldn) > (size_t(4) << 30)) return 0;
   if (!ctx->resident_res) {
     void* h = nullptr;
     RWIG_CUDA_TRY(cudaHostAlloc(&h, sizeof(double) * kResWords, cudaHostAllocMapped));
@@ -725,13 +774,13 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   double* dres = nullptr;
   RWIG_CUDA_TRY(cudaHostGetDevicePointer((void**)&dres, ctx->resident_res, 0));
   const size_t nc = 2 * (size_t)s.gr * N, nrp = 2 * (size_t)s.gc * M;
-  const size_t bytes = sizeof(Packet) * (nc + nrp + 10 * G);
+  const size_t bytes = sizeof(Packet) * (nc + nrp + 14 * G);
   const bool fresh = (int)ctx->slots.size() <= SRS_PACKETS || ctx->slot_bytes[SRS_PACKETS] < bytes;
   Packet* pk = (Packet*)scratch(ctx, SRS_PACKETS, bytes);
   double* info = (double*)scratch(ctx, SRS_INFO, sizeof(double) * 4);
   double* uh = grad ? (double*)scratch(ctx, SRS_UH, 8 * L2 * G * s.ldm) : nullptr;
   double* vh = grad ? (double*)scratch(ctx, SRS_VH, 8 * L2 * G * s.ldn) : nullptr;
-  if (!pk || !info || (grad && (!uh || !vh))) return RWIG_E_NOMEM;
+  if (!pk || !info || (grad && (!uh || !vh))) return 0;
   if (fresh)  // no packet of an earlier life of this memory may carry a tag to come
     RWIG_CUDA_TRY(cudaMemsetAsync(pk, 0, ctx->slot_bytes[SRS_PACKETS], st));
   Args p{};
@@ -761,7 +810,7 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   p.cpart = pk;
   p.rpart = p.cpart + nc;
   p.epart = p.rpart + nrp;
-  p.fin = p.epart + 4 * G;
+  p.fin = p.epart + 8 * G;
   p.epoch = ++ctx->resident_epoch << 32;
   p.res = dres;
   p.err = (unsigned*)(info + 3);
@@ -769,7 +818,7 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   res[kResStatus] = kResRunning;
   res[kResKerr] = 0.0;
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev0, st));
-  masses_kernel<<<1, NTT, 0, st>>>(a, b, M, N, info, p.err);
+  masses_kernel<<<1, kThreads, 0, st>>>(a, b, M, N, info, p.err);
   int rc;
   if (grad) rc = s.reg ? launch<true, true>(p, s, st) : launch<true, false>(p, s, st);
   else rc = s.reg ? launch<false, true>(p, s, st) : launch<false, false>(p, s, st);

@@ -1,0 +1,88 @@
+"""Solves that run whole in one launch with the kernel matrix on the chip
+(sinkhorn_resident.cu) at the edges of their blocks, against the CPU oracle and
+against the general drivers, and the calls they hand back."""
+import numpy as np
+import pytest
+
+import oracle
+import rwig_b200 as rw
+from rwig_b200 import synth
+from tests.util import PARITY_TOL, dual_scale, rel_err
+
+pytestmark = pytest.mark.gpu
+
+ORACLE = {"vanilla": oracle.sinkhorn_vanilla, "log": oracle.sinkhorn_log}
+RESIDENT_LAUNCHES = 2  # the masses and the solve
+
+
+def _problem(m, n, zeros=False):
+    a, b, C = synth.sinkhorn_problem(m, n, 1.0, salt=3 * m + n)
+    if zeros:
+        a[::3] = 0.0
+        b[n // 2:n // 2 + 2] = 0.0
+        a, b = a / a.sum(), b / b.sum()
+    return a, b, C
+
+
+def _same(got, ref, reg, method):
+    assert got["iter"] == ref["iter"]
+    assert got["return_status"] == ref["return_status"]
+    assert rel_err(got["P"], ref["P"]) <= PARITY_TOL
+    assert abs(got["loss"] - ref["loss"]) <= PARITY_TOL * abs(ref["loss"])
+    gs = max(float(np.abs(ref["grad_a"]).max()), abs(ref["loss"]))
+    assert rel_err(got["grad_a"], ref["grad_a"], gs) <= PARITY_TOL
+
+
+# one block and its largest side, one row or column more, thin problems in both
+# directions, the most rows, an odd leading dimension, columns in registers (2048)
+@pytest.mark.parametrize("m,n,zeros", [
+    (3, 2, False), (65, 33, True), (480, 7, False), (481, 480, True), (1, 700, False), (700, 1, False),
+    (2, 9000, False), (8192, 3, False), (1223, 1999, True), (2048, 2048, False),
+])
+@pytest.mark.parametrize("method", ["vanilla", "log"])
+def test_blocks(method, m, n, zeros):
+    a, b, C = _problem(m, n, zeros)
+    par = {"reg": 0.2, "method": method, "with_grad": True, "max_iter": 7, "zero_tol": 1e-13}
+    got = rw.sinkhorn(a, b, C, par)
+    assert rw.last_report()["kernel_launches"] == RESIDENT_LAUNCHES
+    ref = ORACLE[method](a, b, C, 0.2, with_grad=True, max_iter=7, zero_tol=1e-13)
+    _same(got, ref, 0.2, method)
+    assert rw.last_report()["support_m"] == int((a != 0).sum())
+
+
+@pytest.mark.parametrize("m,n,reg", [(300, 500, 0.05), (700, 40, 0.01), (150, 1100, 0.004)])
+def test_general_path_agrees(m, n, reg):
+    """The log method with absorption (log_sinkhorn.tau below its default) runs
+    in the general drivers: same iterations, potentials and gradient."""
+    a, b, C = _problem(m, n, True)
+    par = {"reg": reg, "method": "log", "with_grad": True, "max_iter": 60}
+    got = rw.sinkhorn(a, b, C, par)
+    resident = rw.last_report()["kernel_launches"]
+    L = rw.load()
+    L.rwig_set_option(b"log_sinkhorn.tau", 99.0)
+    try:
+        ref = rw.sinkhorn(a, b, C, par)
+    finally:
+        L.rwig_set_option(b"log_sinkhorn.tau", 100.0)
+    assert resident == RESIDENT_LAUNCHES and rw.last_report()["kernel_launches"] != RESIDENT_LAUNCHES
+    _same(got, ref, reg, "log")
+    on, om = b != 0.0, a != 0.0
+    sc = dual_scale(ref["f"][om], ref["g"][on])
+    assert np.abs(got["f"][om] - ref["f"][om]).max() <= PARITY_TOL * sc
+    assert np.abs(got["g"][on] - ref["g"][on]).max() <= PARITY_TOL * sc
+
+
+@pytest.mark.parametrize("reg,grad", [(1e-3, True), (1.4e-3, False)])
+def test_handed_back(reg, grad):
+    """A kernel matrix with entries below the normal range goes to the general
+    drivers; an underflowed plan entry gives the reference's NaN gradient."""
+    a, b, C = _problem(90, 70)
+    assert C.max() / reg > 709.0
+    par = {"reg": reg, "method": "log", "with_grad": grad, "max_iter": 30}
+    got = rw.sinkhorn(a, b, C, par)
+    assert rw.last_report()["kernel_launches"] != RESIDENT_LAUNCHES
+    ref = oracle.sinkhorn_log(a, b, C, reg, with_grad=grad, max_iter=30)
+    assert got["iter"] == ref["iter"] and got["return_status"] == ref["return_status"]
+    assert rel_err(got["P"], ref["P"]) <= PARITY_TOL
+    if grad:
+        assert rel_err(got["grad_a"], ref["grad_a"]) <= PARITY_TOL
