@@ -25,18 +25,26 @@
 //   grad_A += Fbar / A,  grad_w -= m_l^T logbbar,  then grad_A *= eps, grad_w /= eps.
 // The histories F_l, G_l, m_l, r_l (l = 0..L) stay on the device.
 //
-// Pass kernel: a CTA owns 64 outputs x 16 histograms and one slice of the
-// reduction axis; the 32 x 64 tile of C and the 32 x 16 tile of the
-// potential sit in shared memory, each thread holds 2 x 2 outputs (4
-// exponentials per 4 shared loads).  Partial (max, sum) pairs per slice are
-// merged in a fixed order by the merge kernels, which also carry the
-// elementwise updates above: results are bitwise repeatable.  The
-// exponential is the table method of fastexp.cuh; it is FP64-pipe bound.
+// Pass kernel: a CTA owns one output and all its histograms; lanes run along
+// the reduction axis, which is the contiguous one of C or, for the row passes,
+// of a transposed copy made once per call.  So a sum is complete in its CTA,
+// which carries the elementwise updates above as well: two launches per
+// iteration in each direction, nothing merged between CTAs, every sum in a
+// fixed order (results are bitwise repeatable).  The exponential is the table
+// method of fastexp.cuh.  Large problems are bound by instruction issue (about
+// 26 of them per exponential, 14 in FP64): 2048 x 2048 x 32 takes 355 us a pass.
+// Small ones are bound by one CTA's chain (two loads from L2, the exponentials,
+// two warp reductions, log: 3 us) and the launch: programmatic launches let the
+// next pass's CTAs stand by.  360 x 360 x 5, 20 iterations with gradient: 640 us
+// a call, 7.5 us a pass; with 64 x 16 output tiles and slices of the reduction
+// axis merged by another kernel, 18 CTAs in all there, it took 6047 us, and 8039
+// against 7144 us for 5 iterations of 2048 x 2048 x 32.
 #include <algorithm>
 #include <cmath>
 #include <vector>
 
 #include "barycenter.h"
+#include "common.cuh"
 #include "dgemm.cuh"
 #include "engine.h"
 #include "fastexp.cuh"
@@ -44,239 +52,225 @@
 namespace rwig {
 namespace barylog {
 
-constexpr int TK = 32;   // reduction rows per shared tile
-constexpr int TO = 64;   // outputs per CTA
-constexpr int TS = 16;   // histograms per CTA
-constexpr int NT = 256;  // 32 output groups x 8 histogram pairs
+constexpr int kMaxWarps = 16;  // per CTA
+constexpr int kChunk = 4;      // reduction elements a lane holds at once
+constexpr int kSpread = 4;     // replicas of the exponential's table
 
-// One pass: for outputs o < O, histograms s < S and k in this CTA's slice,
-//   forward  (WEIGHTED = false): max_k x and sum_k exp(x - max), x = (P_ks - C(k,o)) / eps;
-//   weighted (WEIGHTED = true):  sum_k exp((P_ks + Q_os - C(k,o)) / eps) Y_ks,
-// with C(k,o) = C_ko (column pass, k a row of C) or C_ok (row pass, ROWS).
-// P = P1 + p2c P2 (P2 null, or ldp2 = 0 to add a K-vector to every column).
+enum Mode { kColFwd, kRowFwd, kColBwd, kRowBwd };
+
+// One pass over the outputs o < O, histograms s < S, k < K, with C(k,o) at
+// C[k + o K]:
+//   forward   t_os = -eps log sum_k exp((P_ks - C(k,o)) / eps),
+//   backward  t_os = sum_k exp((P_ks + Q_os - C(k,o)) / eps) Y_ks,
+// then the mode's updates (kColFwd: o = j, the new m, logb, G; kRowFwd: o = i,
+// r = t, KV = r - F, the next F and, when D is given, the residual; kColBwd:
+// Gbar = -t and the row step's right-hand side; kRowBwd: Fbar = t, grad_A).
 struct Pass {
   const double* C;
-  long long ldc;
   int K, O, S;
-  const double* P1;
-  long long ldp1;
-  const double* P2;
-  long long ldp2;
-  double p2c;
-  const double* Q;  // O x S (weighted)
-  long long ldq;
-  const double* Y;  // K x S (weighted)
-  long long ldy;
-  double inv_eps;
-  int kchunk;    // reduction rows per slice (a multiple of TK)
-  double* pmax;  // [slices][S][O] (forward)
-  double* psum;  // [slices][S][O]
+  int sw, kw;  // warps along the histograms and along k
+  double eps, inv_eps;
+  const double* P;   // K x S
+  const double* Q;   // O x S (backward)
+  const double* Y;   // K x S (backward)
+  const double* w;   // S
+  double* out;       // O x S: m, r, y, Fbar
+  const double* in;  // O x S: -, F, m, A
+  double* x1;        // O x S: G, the next F, gwp (S x O), grad_A
+  double* logb;      // O (kColFwd)
+  const double* logA;  // O x S (kRowFwd)
+  double* D;           // (kRowFwd)
+  long long ldd;
 };
 
-// exp(x) by the table method, exactly 0 below -708 (where the table method
-// returns its clamp value exp(-708)).
+// exp(x) by the table method for x <= 709, 0 below -708 and for NaN: what the
+// method makes of those is thrown away, which takes a third of the
+// instructions of clamping them first.
 __device__ __forceinline__ double expz(double x, const double* tbl) {
-  const double e = exp_tbl<kExpTableSpread>(x, tbl);
-  return x < -708.0 ? 0.0 : e;
+  const double e = exp_tbl<kSpread, false>(x, tbl);
+  return x >= -708.0 ? e : 0.0;
 }
 
-template <bool ROWS, bool WEIGHTED>
-__global__ void __launch_bounds__(NT) pass_kernel(Pass a) {
-  constexpr int LD = ROWS ? (TO + 2) : (TK + 1);  // shared C tile: ROWS [k][o], else [o][k]
-  __shared__ double ct[ROWS ? TK * (TO + 2) : TO * (TK + 1)];
-  __shared__ double pt[TS * TK];
-  __shared__ double yt[WEIGHTED ? TS * TK : 1];
-  __shared__ double tbl_all[64 * kExpTableSpread];
-  const int tid = threadIdx.x, og = tid & 31, sg = tid >> 5;
-  const int o0 = blockIdx.x * TO, s0 = blockIdx.y * TS;
-  const int kb = blockIdx.z * a.kchunk, ke = min(a.K, kb + a.kchunk);
-  load_exp_table_spread(tbl_all);
-  const double* tbl = tbl_all + (tid & (kExpTableSpread - 1));
+__device__ __forceinline__ double warp_max(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double x = __shfl_xor_sync(0xffffffffu, v, o);
+    v = x > v ? x : v;
+  }
+  return v;
+}
+
+// SQ histograms per warp share each load of C.
+template <int MODE, int SQ>
+__global__ void __launch_bounds__(32 * kMaxWarps, 2) pass_kernel(Pass a) {
+  constexpr bool FWD = MODE == kColFwd || MODE == kRowFwd;
+  constexpr int CH = kChunk;
+  extern __shared__ double part[];  // [kw][S] sums, then (forward) [kw][S] maxima
+  __shared__ double tbl_all[64 * kSpread];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int S = a.S, K = a.K, O = a.O;
+  for (int i = tid; i < 64 * kSpread; i += blockDim.x) tbl_all[i] = __longlong_as_double((long long)kExp2J64[i / kSpread]);
+  const double* tbl = tbl_all + (tid & (kSpread - 1));
   const double ie = a.inv_eps;
-  const int oo[2] = {og, og + 32};
-  const int ss[2] = {2 * sg, 2 * sg + 1};
-  double mx[2][2], sm[2][2], qv[2][2];
-#pragma unroll
-  for (int p = 0; p < 2; ++p)
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      mx[p][q] = -INFINITY;
-      sm[p][q] = 0.0;
-      qv[p][q] = 0.0;
-      if (WEIGHTED && o0 + oo[p] < a.O && s0 + ss[q] < a.S)
-        qv[p][q] = a.Q[(long long)(o0 + oo[p]) + (long long)(s0 + ss[q]) * a.ldq] * ie;
+  const int si = wid % a.sw, ki = wid / a.sw, step = 32 * a.kw;
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the kernel before has ended
+  for (int o = blockIdx.x; o < O; o += gridDim.x) {
+    __syncthreads();  // the table is loaded; the last output's partials are read
+    const double* Co = a.C + (size_t)o * K;
+    // what the updates of histogram tid need, on its way meanwhile
+    double in0 = 0.0, la0 = 0.0;
+    if (MODE != kColFwd && tid < S) {
+      in0 = a.in[o + (size_t)tid * O];
+      if (MODE == kRowFwd) la0 = a.logA[o + (size_t)tid * O];
     }
-  for (int kt = kb; kt < ke; kt += TK) {
-    const int nk = min(TK, ke - kt);
-    __syncthreads();  // the previous tile is consumed (and the table loaded)
-    if (ROWS) {
-      for (int e = tid; e < TK * TO; e += NT) {
-        const int kk = e / TO, o = e % TO;
-        ct[kk * LD + o] = (kk < nk && o0 + o < a.O) ? a.C[(long long)(o0 + o) + (long long)(kt + kk) * a.ldc] : 0.0;
+    for (int s0 = si * SQ; s0 < S; s0 += a.sw * SQ) {
+      double mx[SQ], sm[SQ], qv[SQ];
+      const double* P[SQ];
+      const double* Y[SQ];
+#pragma unroll
+      for (int q = 0; q < SQ; ++q) {
+        const int s = min(s0 + q, S - 1);
+        P[q] = a.P + (size_t)s * K;
+        Y[q] = FWD ? nullptr : a.Y + (size_t)s * K;
+        qv[q] = FWD ? 0.0 : a.Q[o + (size_t)s * O] * ie;
+        mx[q] = -INFINITY;
+        sm[q] = 0.0;
       }
-    } else {
-      for (int e = tid; e < TK * TO; e += NT) {
-        const int o = e / TK, kk = e % TK;
-        ct[o * LD + kk] = (kk < nk && o0 + o < a.O) ? a.C[(long long)(kt + kk) + (long long)(o0 + o) * a.ldc] : 0.0;
+      for (int kb = 32 * ki; kb < K; kb += CH * step) {
+        // elements beyond K: C = inf, which contributes nothing; whole warps
+        // beyond it are skipped
+        double x[SQ][CH], y[FWD ? 1 : SQ][CH];
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+          const int k = kb + i * step + lane;
+          const bool in = k < K;
+          const double c = in ? Co[k] : INFINITY;
+#pragma unroll
+          for (int q = 0; q < SQ; ++q) {
+            x[q][i] = ((in ? P[q][k] : 0.0) - c) * ie;
+            if (!FWD) y[q][i] = in ? Y[q][k] : 0.0;
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < SQ; ++q) {
+          if (FWD) {
+            double tm = mx[q];
+#pragma unroll
+            for (int i = 0; i < CH; ++i) tm = x[q][i] > tm ? x[q][i] : tm;
+            if (tm > mx[q]) {
+              if (kb >= CH * step) sm[q] *= expz(mx[q] - tm, tbl);
+              mx[q] = tm;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < CH; ++i)
+            if (kb + i * step < K) {
+              if (FWD) {
+                sm[q] += expz(x[q][i] - mx[q], tbl);
+              } else {
+                const double z = x[q][i] + qv[q];
+                sm[q] = fma(expz(z > 709.0 ? 709.0 : z, tbl), y[q][i], sm[q]);
+              }
+            }
+        }
       }
-    }
-    for (int e = tid; e < TS * TK; e += NT) {
-      const int s = e / TK, kk = e % TK;
-      double v = 0.0, y = 0.0;
-      if (kk < nk && s0 + s < a.S) {
-        const long long k = kt + kk;
-        v = a.P1[k + (long long)(s0 + s) * a.ldp1];
-        if (a.P2) v += a.p2c * a.P2[k + (long long)(s0 + s) * a.ldp2];
-        if (WEIGHTED) y = a.Y[k + (long long)(s0 + s) * a.ldy];
+#pragma unroll
+      for (int q = 0; q < SQ; ++q) {
+        double m = 0.0, t = sm[q];
+        if (FWD) {
+          m = warp_max(mx[q]);
+          t *= exp(mx[q] - m);
+        }
+        t = warp_sum(t);
+        if (lane == 0 && s0 + q < S) {
+          part[ki * S + s0 + q] = t;
+          if (FWD) part[(a.kw + ki) * S + s0 + q] = m;
+        }
       }
-      pt[s * TK + kk] = v;
-      if (WEIGHTED) yt[s * TK + kk] = y;
     }
     __syncthreads();
-    const double* c0p = ROWS ? ct + oo[0] : ct + oo[0] * LD;
-    const double* c1p = ROWS ? ct + oo[1] : ct + oo[1] * LD;
-    constexpr int CK = ROWS ? LD : 1;  // stride of k in the C tile
-    const double* p0p = pt + ss[0] * TK;
-    const double* p1p = pt + ss[1] * TK;
-    if (!WEIGHTED) {
-      double tm[2][2] = {{-INFINITY, -INFINITY}, {-INFINITY, -INFINITY}};
-      for (int kk = 0; kk < nk; ++kk) {
-        const double c0 = c0p[kk * CK], c1 = c1p[kk * CK], p0 = p0p[kk], p1 = p1p[kk];
-        tm[0][0] = fmax(tm[0][0], (p0 - c0) * ie);
-        tm[0][1] = fmax(tm[0][1], (p1 - c0) * ie);
-        tm[1][0] = fmax(tm[1][0], (p0 - c1) * ie);
-        tm[1][1] = fmax(tm[1][1], (p1 - c1) * ie);
-      }
-#pragma unroll
-      for (int p = 0; p < 2; ++p)
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-          if (tm[p][q] > mx[p][q]) {
-            sm[p][q] *= expz(mx[p][q] - tm[p][q], tbl);
-            mx[p][q] = tm[p][q];
-          }
-      for (int kk = 0; kk < nk; ++kk) {
-        const double c0 = c0p[kk * CK], c1 = c1p[kk * CK], p0 = p0p[kk], p1 = p1p[kk];
-        sm[0][0] += expz((p0 - c0) * ie - mx[0][0], tbl);
-        sm[0][1] += expz((p1 - c0) * ie - mx[0][1], tbl);
-        sm[1][0] += expz((p0 - c1) * ie - mx[1][0], tbl);
-        sm[1][1] += expz((p1 - c1) * ie - mx[1][1], tbl);
-      }
-    } else {
-      const double* y0p = yt + ss[0] * TK;
-      const double* y1p = yt + ss[1] * TK;
-      for (int kk = 0; kk < nk; ++kk) {
-        const double c0 = c0p[kk * CK], c1 = c1p[kk * CK], p0 = p0p[kk], p1 = p1p[kk];
-        const double y0 = y0p[kk], y1 = y1p[kk];
-        sm[0][0] = fma(expz((p0 - c0) * ie + qv[0][0], tbl), y0, sm[0][0]);
-        sm[0][1] = fma(expz((p1 - c0) * ie + qv[0][1], tbl), y1, sm[0][1]);
-        sm[1][0] = fma(expz((p0 - c1) * ie + qv[1][0], tbl), y0, sm[1][0]);
-        sm[1][1] = fma(expz((p1 - c1) * ie + qv[1][1], tbl), y1, sm[1][1]);
-      }
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < 2; ++p)
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int o = o0 + oo[p], s = s0 + ss[q];
-      if (o < a.O && s < a.S) {
-        const long long idx = ((long long)blockIdx.z * a.S + s) * a.O + o;
-        if (!WEIGHTED) a.pmax[idx] = mx[p][q];
-        a.psum[idx] = sm[p][q];
-      }
-    }
-}
-
-// Merged soft-min of output o, histogram s over the slices (fixed order):
-// -eps (max + log sum_slices psum exp(pmax - max)).
-__device__ __forceinline__ double merged_softmin(const double* pmax, const double* psum, int slices, int S, int O,
-                                                 int s, int o, double eps) {
-  double mx = -INFINITY;
-  for (int z = 0; z < slices; ++z) mx = fmax(mx, pmax[((long long)z * S + s) * O + o]);
-  double sum = 0.0;
-  for (int z = 0; z < slices; ++z) {
-    const long long k = ((long long)z * S + s) * O + o;
-    sum += psum[k] * exp(pmax[k] - mx);
-  }
-  return -eps * (mx + log(sum));
-}
-
-// Forward, after the column pass over C - F_l (thread per support point j):
-// m_l (into Mh), logb_j = -(sum_s w_s m_js) / eps, G_l = eps logb + m.
-__global__ void col_merge_fwd(const double* pmax, const double* psum, int slices, int N, int S, double eps,
-                              const double* w, double* M_out, double* G, double* logb) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < N; j += gridDim.x * blockDim.x) {
+    // totals over the k warps, and the updates; threads s < S (one warp for the
+    // column modes, which also sum over s)
+    constexpr bool COL = MODE == kColFwd || MODE == kColBwd;
     double acc = 0.0;
-    for (int s = 0; s < S; ++s) {
-      const double m = merged_softmin(pmax, psum, slices, S, N, s, j, eps);
-      M_out[j + (long long)s * N] = m;
-      acc += m * w[s];
+    const int ns = COL ? 32 : (int)blockDim.x;
+    if (tid < ns)
+      for (int s = tid; s < S; s += ns) {
+        double t = 0.0;
+        if (FWD) {
+          double m = -INFINITY;
+          for (int z = 0; z < a.kw; ++z) m = fmax(m, part[(a.kw + z) * S + s]);
+          if (a.kw == 1) t = part[s];
+          else
+            for (int z = 0; z < a.kw; ++z) t += part[z * S + s] * exp(part[(a.kw + z) * S + s] - m);
+          t = -a.eps * (m + log(t));
+        } else {
+          for (int z = 0; z < a.kw; ++z) t += part[z * S + s];
+        }
+        const size_t e = o + (size_t)s * O;
+        if (MODE == kColFwd) {
+          a.out[e] = t;
+          part[s] = t;  // (this thread alone reads column s of the partials)
+          acc += t * a.w[s];
+        } else if (MODE == kRowFwd) {
+          const double f = s == tid ? in0 : a.in[e], kv = t - f, la = s == tid ? la0 : a.logA[e];
+          a.out[e] = t;
+          a.x1[e] = f + (a.eps * la + kv);                                   // :231
+          if (a.D) a.D[o + (long long)s * a.ldd] = -kv / a.eps - la;         // :252
+        } else if (MODE == kColBwd) {
+          part[s] = -t;
+          acc -= t;
+        } else {
+          a.out[e] = t;
+          a.x1[e] += t / (s == tid ? in0 : a.in[e]);
+        }
+      }
+    if (COL && tid < 32) {
+      acc = warp_sum(acc);
+      if (MODE == kColFwd) {
+        const double lb = -acc / a.eps;  // barycenter_impl_log.cpp:239
+        if (lane == 0) a.logb[o] = lb;
+        for (int s = lane; s < S; s += 32) a.x1[o + (size_t)s * O] = a.eps * lb + part[s];  // :245
+      } else {
+        const double lbb = a.eps * acc;
+        for (int s = lane; s < S; s += 32) {
+          a.out[o + (size_t)s * O] = (a.w[s] / a.eps) * lbb - part[s];
+          a.x1[(size_t)o * S + s] -= (s == tid ? in0 : a.in[o + (size_t)s * O]) * lbb;  // :368-372
+        }
+      }
     }
-    const double lb = -acc / eps;  // barycenter_impl_log.cpp:239
-    logb[j] = lb;
-    for (int s = 0; s < S; ++s) G[j + (long long)s * N] = eps * lb + M_out[j + (long long)s * N];  // :245
   }
 }
 
-// Forward, after the row pass over C - G (thread per (i, s)): r (into R_out
-// when given), KV = r - F, the next F = F + (eps log A + KV) (:231) and, when
-// D is given, the stopping residual -KV / eps - log A (:252).
-__global__ void row_merge_fwd(const double* pmax, const double* psum, int slices, int M, int S, double eps,
-                              const double* F, const double* logA, double* R_out, double* Fnext, double* D,
-                              long long ldd) {
-  const long long n = (long long)M * S;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % M), s = (int)(e / M);
-    const double r = merged_softmin(pmax, psum, slices, S, M, s, i, eps);
-    const double kv = r - F[e];
-    if (R_out) R_out[e] = r;
-    Fnext[e] = F[e] + (eps * logA[e] + kv);
-    if (D) D[i + (long long)s * ldd] = -kv / eps - logA[e];
-  }
-}
-
-// Adjoint seed and column step (thread per support point j).  seed: logbbar
-// = 2 (b - b_ext) o b with the normalised b (:324), Gbar = 0; otherwise
-// Gbar_js = -(sum over slices of the weighted pass), logbbar = eps sum_s Gbar.
-// Then y = (w / eps) logbbar - Gbar (the right-hand side of the row step) and
-// gwp[j S + s] -= m_l,js logbbar_j (:368-372).
-__global__ void col_merge_bwd(const double* psum, int slices, int N, int S, double eps, int seed, const double* bn,
-                              const double* bext, const double* w, const double* Ml, double* Yv, double* gwp) {
+// Adjoint seed (thread per support point j): logbbar = 2 (b - b_ext) o b with
+// the normalised b (:324), Gbar = 0, y = (w / eps) logbbar, gwp[j S + s] =
+// -m_L,js logbbar_j.
+__global__ void seed_bwd(int N, int S, double eps, const double* bn, const double* bext, const double* w,
+                         const double* Ml, double* Yv, double* gwp) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < N; j += gridDim.x * blockDim.x) {
-    double lbb;
-    if (seed) {
-      lbb = 2.0 * (bn[j] - bext[j]) * bn[j];
-      for (int s = 0; s < S; ++s) Yv[j + (long long)s * N] = (w[s] / eps) * lbb;
-    } else {
-      double acc = 0.0;
-      for (int s = 0; s < S; ++s) {
-        double g = 0.0;
-        for (int z = 0; z < slices; ++z) g += psum[((long long)z * S + s) * N + j];
-        g = -g;
-        Yv[j + (long long)s * N] = g;  // Gbar, replaced by y below
-        acc += g;
-      }
-      lbb = eps * acc;
-      for (int s = 0; s < S; ++s) {
-        const long long k = j + (long long)s * N;
-        Yv[k] = (w[s] / eps) * lbb - Yv[k];
-      }
+    const double lbb = 2.0 * (bn[j] - bext[j]) * bn[j];
+    for (int s = 0; s < S; ++s) {
+      Yv[j + (long long)s * N] = (w[s] / eps) * lbb;
+      gwp[(long long)j * S + s] -= Ml[j + (long long)s * N] * lbb;
     }
-    for (int s = 0; s < S; ++s) gwp[(long long)j * S + s] -= Ml[j + (long long)s * N] * lbb;
   }
 }
 
-// Adjoint row step (thread per (i, s)): Fbar = sum over slices; grad_A += Fbar / A.
-__global__ void row_merge_bwd(const double* psum, int slices, int M, int S, const double* A, double* Fbar,
-                              double* gA) {
-  const long long n = (long long)M * S;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % M), s = (int)(e / M);
-    double f = 0.0;
-    for (int z = 0; z < slices; ++z) f += psum[((long long)z * S + s) * M + i];
-    Fbar[e] = f;
-    gA[e] += f / A[e];
+// Ct (N x M) = the transpose of C (M x N), 32 x 32 tiles.
+__global__ void __launch_bounds__(256) transpose_kernel(const double* C, int M, int N, double* Ct) {
+  __shared__ double t[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int tm = (M + 31) / 32;
+  const long long tiles = (long long)tm * ((N + 31) / 32);
+  for (long long b = blockIdx.x; b < tiles; b += gridDim.x) {
+    const int m0 = (int)(b % tm) * 32, n0 = (int)(b / tm) * 32;
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8)
+      if (m0 + tx < M && n0 + r < N) t[r][tx] = C[(size_t)(n0 + r) * M + m0 + tx];
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8)
+      if (n0 + tx < N && m0 + r < M) Ct[(size_t)(m0 + r) * N + n0 + tx] = t[tx][r];
   }
 }
 
@@ -345,7 +339,7 @@ __global__ void finish_b(const double* logb, int N, const double* bext, double* 
 }
 
 enum {
-  SL_FH = 300, SL_GH, SL_MH, SL_RH, SL_LB, SL_LOGA, SL_D, SL_GRAM, SL_PMAX, SL_PSUM, SL_FBAR, SL_Y, SL_GA,
+  SL_FH = 300, SL_GH, SL_MH, SL_RH, SL_LB, SL_LOGA, SL_D, SL_GRAM, SL_CT, SL_FBAR, SL_Y, SL_GA,
   SL_GWP, SL_GW, SL_BN, SL_SCAL
 };
 
@@ -353,12 +347,35 @@ int grid1(const Context* ctx, long long n) {
   return (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 8LL * ctx->sm_count));
 }
 
-// Reduction slices for a pass with `tiles` CTAs per slice: about two CTAs
-// per SM in all, each slice at least 4 shared tiles long.
-int pick_slices(const Context* ctx, long long tiles, int K) {
-  const long long want = (2LL * ctx->sm_count + tiles - 1) / tiles;
-  const long long most = std::max(1, (K + 4 * TK - 1) / (4 * TK));
-  return (int)std::max(1LL, std::min(want, most));
+// Launch of a pass.  Histograms per warp: one up to 8 of them (more warps),
+// else two, which read C half as often (2048 x 2048 x 32: 1421 us per iteration
+// and its backward step against 1607 with one and 1460 with four, which need
+// 128 registers).  Warps along k: until the chip has 16 warps per SM or a lane
+// has one chunk (360 x 360 x 5: 838 us a call against 922 with 8 warps per SM).
+template <int MODE>
+void launch_pass(const Context* ctx, Pass a, cudaStream_t st) {
+  const int sq = a.S <= 8 ? 1 : 2;
+  a.sw = std::min(8, (a.S + sq - 1) / sq);
+  a.kw = 1;
+  while (2 * a.kw * a.sw <= kMaxWarps && 32LL * kChunk * a.kw < a.K &&
+         (long long)a.O * a.sw * a.kw < 16LL * ctx->sm_count)
+    a.kw *= 2;
+  const int threads = 32 * a.sw * a.kw;
+  const int grid = (int)std::min<long long>(a.O, (long long)ctx->sm_count * (2048 / threads));
+  const size_t smem = sizeof(double) * 2 * (size_t)a.kw * a.S;  // at most 16 KB (64 histograms)
+  // the next pass may take its place while this one drains (it waits for its
+  // end before it reads anything)
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, sq == 1 ? pass_kernel<MODE, 1> : pass_kernel<MODE, 2>, a);  // (errors: at the next check)
 }
 
 }  // namespace barylog
@@ -378,14 +395,6 @@ int run_log(Context* ctx, cudaStream_t st, double* X1, double* X2, double* b, do
   const long long ldd = ((M + 1) / 2) * 2;
   const int H = withgrad ? L + 2 : 2;  // slots of F (l = 0..L+1) and of G, m, r
   const bool fixed = !(tol > 0.0);
-  // slices of the passes (the column passes reduce over M, the row passes over N)
-  const long long col_tiles = (long long)((N + TO - 1) / TO) * ((S + TS - 1) / TS);
-  const long long row_tiles = (long long)((M + TO - 1) / TO) * ((S + TS - 1) / TS);
-  const int zc = pick_slices(ctx, col_tiles, M), zr = pick_slices(ctx, row_tiles, N);
-  const int kc_col = ((M + zc - 1) / zc + TK - 1) / TK * TK, kc_row = ((N + zr - 1) / zr + TK - 1) / TK * TK;
-  const int zcol = (M + kc_col - 1) / kc_col, zrow = (N + kc_row - 1) / kc_row;
-  const size_t part = std::max((size_t)zcol * NS, (size_t)zrow * MS);
-
   double* Fh = (double*)scratch(ctx, SL_FH, sizeof(double) * MS * H);
   double* Gh = (double*)scratch(ctx, SL_GH, sizeof(double) * NS * H);
   double* Mh = (double*)scratch(ctx, SL_MH, sizeof(double) * NS * H);
@@ -394,11 +403,10 @@ int run_log(Context* ctx, cudaStream_t st, double* X1, double* X2, double* b, do
   double* logA = (double*)scratch(ctx, SL_LOGA, sizeof(double) * MS);
   double* D = (double*)scratch(ctx, SL_D, sizeof(double) * ldd * S);
   double* gram = (double*)scratch(ctx, SL_GRAM, sizeof(double) * S * S);
-  double* pmax = (double*)scratch(ctx, SL_PMAX, sizeof(double) * part);
-  double* psum = (double*)scratch(ctx, SL_PSUM, sizeof(double) * part);
+  double* Ct = (double*)scratch(ctx, SL_CT, sizeof(double) * (size_t)M * N);
   double* bn = (double*)scratch(ctx, SL_BN, sizeof(double) * N);
   double* scal = (double*)scratch(ctx, SL_SCAL, sizeof(double) * 8);
-  if (!Fh || !Gh || !Mh || !Rh || !lb || !logA || !D || !gram || !pmax || !psum || !bn || !scal) return RWIG_E_NOMEM;
+  if (!Fh || !Gh || !Mh || !Rh || !lb || !logA || !D || !gram || !Ct || !bn || !scal) return RWIG_E_NOMEM;
   double *Fbar = nullptr, *Yv = nullptr, *gA = nullptr, *gwp = nullptr, *gw = nullptr;
   if (withgrad) {
     Fbar = (double*)scratch(ctx, SL_FBAR, sizeof(double) * MS);
@@ -411,26 +419,27 @@ int run_log(Context* ctx, cudaStream_t st, double* X1, double* X2, double* b, do
   auto slot = [&](double* base, size_t sz, int l) { return base + sz * (size_t)(withgrad ? l : (l & 1)); };
   const double inv_eps = 1.0 / reg;
   int nl = 0;
-  // column pass over C - P (P: M x S), row pass over C - P (P: N x S)
-  auto col_pass = [&](const double* P1, const double* P2, long long ldp2, double p2c, const double* Q,
-                      const double* Y) -> int {
-    Pass p{C, (long long)M, M, N, S, P1, (long long)M, P2, ldp2, p2c, Q, (long long)N, Y, (long long)M,
-           inv_eps, kc_col, pmax, psum};
-    const dim3 grid((N + TO - 1) / TO, (S + TS - 1) / TS, zcol);
-    if (Y) pass_kernel<false, true><<<grid, NT, 0, st>>>(p);
-    else pass_kernel<false, false><<<grid, NT, 0, st>>>(p);
+  // passes over the columns (o = j, k = i) and the rows (o = i, k = j) of C
+  Pass col{}, row{};
+  col.C = C;
+  col.K = row.O = M;
+  col.O = row.K = N;
+  row.C = Ct;
+  col.S = row.S = S;
+  col.eps = row.eps = reg;
+  col.inv_eps = row.inv_eps = inv_eps;
+  col.w = w;
+  col.logb = lb;
+  row.logA = logA;
+  row.ldd = ldd;
+  auto row_fwd = [&](int l, double* d) {  // r_l, F_{l+1}
+    row.P = slot(Gh, NS, l);
+    row.in = slot(Fh, MS, l);
+    row.out = slot(Rh, MS, l);
+    row.x1 = slot(Fh, MS, l + 1);
+    row.D = d;
+    launch_pass<kRowFwd>(ctx, row, st);
     ++nl;
-    return 0;
-  };
-  auto row_pass = [&](const double* P1, const double* P2, long long ldp2, double p2c, const double* Q,
-                      const double* Y) -> int {
-    Pass p{C, (long long)M, N, M, S, P1, (long long)N, P2, ldp2, p2c, Q, (long long)M, Y, (long long)N,
-           inv_eps, kc_row, pmax, psum};
-    const dim3 grid((M + TO - 1) / TO, (S + TS - 1) / TS, zrow);
-    if (Y) pass_kernel<true, true><<<grid, NT, 0, st>>>(p);
-    else pass_kernel<true, false><<<grid, NT, 0, st>>>(p);
-    ++nl;
-    return 0;
   };
 
   // F_0 = G_0 = 0, log A; the initial row soft-min at (0, 0) gives F_1 (:221, :231)
@@ -439,24 +448,21 @@ int run_log(Context* ctx, cudaStream_t st, double* X1, double* X2, double* b, do
   zero_kernel<<<grid1(ctx, N), 256, 0, st>>>(lb, N);
   log_kernel<<<grid1(ctx, MS), 256, 0, st>>>(A, (long long)MS, logA);
   nl += 4;
-  row_pass(slot(Gh, NS, 0), nullptr, 0, 0.0, nullptr, nullptr);
-  row_merge_fwd<<<grid1(ctx, MS), 256, 0, st>>>(pmax, psum, zrow, M, S, reg, slot(Fh, MS, 0), logA, nullptr,
-                                                  slot(Fh, MS, 1), nullptr, ldd);
+  transpose_kernel<<<std::min(16 * ctx->sm_count, ((M + 31) / 32) * ((N + 31) / 32)), 256, 0, st>>>(C, M, N, Ct);
   ++nl;
+  row_fwd(0, nullptr);
   int iter = 0;
   double err = 1000.0;
   while (iter < L && err >= tol) {
     ++iter;
     const int l = iter;
-    col_pass(slot(Fh, MS, l), nullptr, 0, 0.0, nullptr, nullptr);
-    col_merge_fwd<<<grid1(ctx, N), 256, 0, st>>>(pmax, psum, zcol, N, S, reg, w, slot(Mh, NS, l), slot(Gh, NS, l),
-                                                  lb);
-    row_pass(slot(Gh, NS, l), nullptr, 0, 0.0, nullptr, nullptr);
+    col.P = slot(Fh, MS, l);
+    col.out = slot(Mh, NS, l);
+    col.x1 = slot(Gh, NS, l);
+    launch_pass<kColFwd>(ctx, col, st);
+    ++nl;
     const bool need_err = !fixed || iter == L;
-    row_merge_fwd<<<grid1(ctx, MS), 256, 0, st>>>(pmax, psum, zrow, M, S, reg, slot(Fh, MS, l), logA,
-                                                    slot(Rh, MS, l), slot(Fh, MS, l + 1), need_err ? D : nullptr,
-                                                    ldd);
-    nl += 2;
+    row_fwd(l, need_err ? D : nullptr);
     RWIG_CUDA_TRY(cudaGetLastError());
     if (need_err) {
       int gl = 0;
@@ -477,16 +483,26 @@ int run_log(Context* ctx, cudaStream_t st, double* X1, double* X2, double* b, do
     RWIG_CUDA_TRY(cudaMemsetAsync(gA, 0, sizeof(double) * MS, st));
     RWIG_CUDA_TRY(cudaMemsetAsync(gwp, 0, sizeof(double) * NS, st));
     for (int l = iter; l >= 1; --l) {
-      const bool seed = (l == iter);
-      if (!seed) {
+      if (l == iter) {
+        seed_bwd<<<grid1(ctx, N), 256, 0, st>>>(N, S, reg, bn, bext, w, slot(Mh, NS, l), Yv, gwp);
+      } else {
         // Gbar: column pass weighted by the row softmax at (F_l, G_l) (:306-320)
-        col_pass(slot(Rh, MS, l), nullptr, 0, 0.0, slot(Gh, NS, l), Fbar);
+        col.P = slot(Rh, MS, l);
+        col.Q = slot(Gh, NS, l);
+        col.Y = Fbar;
+        col.out = Yv;
+        col.in = slot(Mh, NS, l);
+        col.x1 = gwp;
+        launch_pass<kColBwd>(ctx, col, st);
       }
-      col_merge_bwd<<<grid1(ctx, N), 256, 0, st>>>(psum, zcol, N, S, reg, seed ? 1 : 0, bn, bext, w,
-                                                    slot(Mh, NS, l), Yv, gwp);
       // Fbar: row pass weighted by the column softmax at (F_l, G_{l-1}) (:330-346)
-      row_pass(slot(Mh, NS, l), nullptr, 0, 0.0, slot(Fh, MS, l), Yv);
-      row_merge_bwd<<<grid1(ctx, MS), 256, 0, st>>>(psum, zrow, M, S, A, Fbar, gA);
+      row.P = slot(Mh, NS, l);
+      row.Q = slot(Fh, MS, l);
+      row.Y = Yv;
+      row.out = Fbar;
+      row.in = A;
+      row.x1 = gA;
+      launch_pass<kRowBwd>(ctx, row, st);
       nl += 2;
     }
     axpby_kernel<<<grid1(ctx, MS), 256, 0, st>>>(gA, (long long)MS, reg);  // :376

@@ -197,6 +197,7 @@ extern "C" void rwig_shutdown(void) {
       if (p) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->resident_res) cudaFreeHost(c->resident_res);
+    if (c->range_res) cudaFreeHost(c->range_res);
     cudaEventDestroy(c->ev0);
     cudaEventDestroy(c->ev1);
     cudaEventDestroy(c->evk);

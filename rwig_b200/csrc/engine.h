@@ -50,6 +50,7 @@ struct Context {
   // whole-solve Sinkhorn launches (sinkhorn_resident.cu): host-mapped results
   // and the number of the last launch, which its packets' tags carry
   double* resident_res = nullptr;
+  double* range_res = nullptr;  // host-mapped: what barycenter.cu's Gibbs kernel found, for a host still enqueuing
   unsigned long long resident_epoch = 0;
   // the K whose INT8 residue planes the scratch holds (oz::prepare_reuse):
   // its size and leading dimension, valid while no other prepare ran

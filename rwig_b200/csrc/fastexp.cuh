@@ -57,13 +57,15 @@ __device__ __forceinline__ void load_exp_table_spread(double* tbl) {
 
 // tbl: the table as laid out by load_exp_table (stride 1) or, with
 // STRIDE = kExpTableSpread, by load_exp_table_spread offset by the lane's replica.
-template <int STRIDE = 1>
+// CLAMP = false leaves out the clamp: the caller replaces the result for x
+// outside [-708, 709].
+template <int STRIDE = 1, bool CLAMP = true>
 __device__ __forceinline__ double exp_tbl(double x, const double* tbl) {
   const double kInvLn2_64 = 92.33248261689366;          // 64 / ln 2
   const double kLn2_64_hi = 0.010830424696249145;       // ln2/64 rounded to double
   const double kLn2_64_lo = 3.623510646634843e-19;      // ln2/64 - kLn2_64_hi
   const double kShifter = 6755399441055744.0;           // 1.5 * 2^52
-  const double xc = fmin(fmax(x, -708.0), 709.0);
+  const double xc = CLAMP ? fmin(fmax(x, -708.0), 709.0) : x;
   const double t = fma(xc, kInvLn2_64, kShifter);
   const int k = __double2loint(t);
   const double kd = t - kShifter;
