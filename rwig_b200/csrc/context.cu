@@ -173,6 +173,12 @@ void* scratch(Context* ctx, int k, size_t bytes) {
   return p;
 }
 
+int ensure_mapped(Context* ctx) {
+  if (!ctx->mapped)
+    RWIG_CUDA_TRY(cudaHostAlloc((void**)&ctx->mapped, sizeof(double) * Context::kMappedWords, cudaHostAllocMapped));
+  return 0;
+}
+
 }  // namespace rwig
 
 using namespace rwig;
@@ -197,7 +203,7 @@ extern "C" void rwig_shutdown(void) {
       if (p) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->resident_res) cudaFreeHost(c->resident_res);
-    if (c->range_res) cudaFreeHost(c->range_res);
+    if (c->mapped) cudaFreeHost(c->mapped);
     cudaEventDestroy(c->ev0);
     cudaEventDestroy(c->ev1);
     cudaEventDestroy(c->evk);

@@ -19,6 +19,12 @@
 // rows then go to an epilogue functor, so the elementwise work that follows
 // each product never makes a separate pass over HBM.
 //
+// What bounds it: 2048 x 2048 x 32 takes 19.5 us (7.6 of arithmetic at the
+// cuBLAS FP64 rate), two CTAs per SM on three quarters of the SMs, the rest
+// spent on filling the ring from L2, the cluster's sum and the epilogue.  Small
+// products are all of the latter: launches are programmatic, so that the next
+// product's CTAs come up, and read K's first tiles, while this one drains.
+//
 // Epilogue interface (called by all NTH threads of the CTA; may use
 // __syncthreads):
 //     epi(r0, nr, c0, nc, t, ldt, ws)
@@ -56,6 +62,7 @@ struct GemmArgs {
   int tcols;         // output columns per tile (<= BN; 0: BN).  A multiple of an
                      // epilogue's column group keeps every group inside one tile.
   int tile0;         // first tile of the launch (wide-tile kernel; 0 otherwise)
+  int early;         // K was not written by the kernel before this one in the stream (see gemm)
 };
 
 template <int TRANS>
@@ -132,12 +139,23 @@ __device__ __forceinline__ double ld_cluster(const double* p, unsigned rank) {
   return v;
 }
 
+// Sum of the partials at p of the first `splits` CTAs, in order, their loads
+// issued together (each takes some 200 clocks).
+__device__ __forceinline__ double sum_cluster(const double* p, int splits) {
+  double x[kMaxSplits], v = 0.0;
+#pragma unroll
+  for (int q = 0; q < kMaxSplits; ++q) x[q] = q < splits ? ld_cluster(p, (unsigned)q) : 0.0;
+#pragma unroll
+  for (int q = 0; q < kMaxSplits; ++q)
+    if (q < splits) v += x[q];
+  return v;
+}
+
 // Issues the copies of contraction step [k0, k0 + BK) into one ring stage.
 // XV = 2: X columns copied as 16-byte pairs (ldx even, X 16-byte aligned);
 // XV = 1: 8-byte copies.  Out-of-range elements are zero-filled.
-template <int TRANS, int NT, int XV, int BMT = BM>
-__device__ __forceinline__ void load_stage(const GemmArgs& g, double* As, double* Bs, int m0, int n0, int tc,
-                                           int k0, int kend) {
+template <int TRANS, int BMT = BM>
+__device__ __forceinline__ void load_a(const GemmArgs& g, double* As, int m0, int k0, int kend) {
   const int tid = threadIdx.x;
   if (!TRANS) {
     // A[k][m] = K[m + k*ldk]: 32 k x BMT/2 m-pairs
@@ -170,6 +188,10 @@ __device__ __forceinline__ void load_stage(const GemmArgs& g, double* As, double
       cp_async16(As + mm * (BK + PAD) + kp, src, bytes);
     }
   }
+}
+template <int NT, int XV>
+__device__ __forceinline__ void load_b(const GemmArgs& g, double* Bs, int n0, int tc, int k0, int kend) {
+  const int tid = threadIdx.x;
   // B[n][k] = X[k + n*ldx]
   if (XV == 2) {
 #pragma unroll
@@ -202,6 +224,35 @@ __device__ __forceinline__ void load_stage(const GemmArgs& g, double* As, double
   }
 }
 
+template <int TRANS, int NT, int XV, int BMT = BM>
+__device__ __forceinline__ void load_stage(const GemmArgs& g, double* As, double* Bs, int m0, int n0, int tc,
+                                           int k0, int kend) {
+  load_a<TRANS, BMT>(g, As, m0, k0, kend);
+  load_b<NT, XV>(g, Bs, n0, tc, k0, kend);
+}
+// The first STG - 1 stages.  The next product of the stream may start while
+// this one drains; it reads nothing written by the kernel before it until that
+// has ended, but K's tiles on `early`.
+template <int TRANS, int NT, int XV, int BMT, int STG, int ASZ, int BSZ>
+__device__ __forceinline__ void load_first(const GemmArgs& g, double* As, double* Bs, int m0, int n0, int tc,
+                                           int kbeg, int kend, int nsteps) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  if (g.early) {
+#pragma unroll
+    for (int s = 0; s < STG - 1; ++s)
+      if (s < nsteps) load_a<TRANS, BMT>(g, As + s * ASZ, m0, kbeg + s * BK, kend);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+  for (int s = 0; s < STG - 1; ++s) {
+    if (s < nsteps) {
+      if (!g.early) load_a<TRANS, BMT>(g, As + s * ASZ, m0, kbeg + s * BK, kend);
+      load_b<NT, XV>(g, Bs + s * BSZ, n0, tc, kbeg + s * BK, kend);
+    }
+    cp_async_commit();
+  }
+}
+
 // KM: k extent of one DMMA instruction (4, 8 or 16).
 template <int TRANS, int NT, int XV, class Epi, int KM>
 __global__ void __launch_bounds__(NTH) dgemm_kernel(GemmArgs g, Epi epi) {
@@ -231,11 +282,7 @@ __global__ void __launch_bounds__(NTH) dgemm_kernel(GemmArgs g, Epi epi) {
 
   double* As = smem;
   double* Bs = smem + STAGES * ASZ;
-#pragma unroll
-  for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < nsteps) load_stage<TRANS, NT, XV>(g, As + s * ASZ, Bs + s * BSZ, m0, n0, tc, kbeg + s * BK, kend);
-    cp_async_commit();
-  }
+  load_first<TRANS, NT, XV, BM, STAGES, ASZ, BSZ>(g, As, Bs, m0, n0, tc, kbeg, kend, nsteps);
   const int wm = (warp & 3) * 16, kh = (warp >> 2) * (BK / 2);
   for (int s = 0; s < nsteps; ++s) {
     cp_async_wait<STAGES - 2>();
@@ -307,13 +354,7 @@ __global__ void __launch_bounds__(NTH) dgemm_kernel(GemmArgs g, Epi epi) {
   for (int e = threadIdx.x; e < rows * BN; e += NTH) {
     const int r = e % rows, c = e / rows;
     const double* p = red + c * (BM + 1) + rl0 + r;
-    double v = 0.0;
-    if (splits > 1) {
-      for (int q = 0; q < splits; ++q) v += ld_cluster(p, (unsigned)q);
-    } else {
-      v += *p;
-    }
-    fin[c * rows + r] = v;
+    fin[c * rows + r] = splits > 1 ? sum_cluster(p, splits) : *p;
   }
   if (splits > 1) cluster_arrive();  // this CTA is done reading its peers
   __syncthreads();
@@ -374,12 +415,7 @@ __global__ void __launch_bounds__(NTH, 1) dgemm2_kernel(GemmArgs g, Epi epi) {
 
   double* As = smem;
   double* Bs = smem + STAGES2 * ASZ;
-#pragma unroll
-  for (int s = 0; s < STAGES2 - 1; ++s) {
-    if (s < nsteps)
-      load_stage<TRANS, NT, XV, BM2>(g, As + s * ASZ, Bs + s * BSZ, m0, n0, tc, kbeg + s * BK, kend);
-    cp_async_commit();
-  }
+  load_first<TRANS, NT, XV, BM2, STAGES2, ASZ, BSZ>(g, As, Bs, m0, n0, tc, kbeg, kend, nsteps);
   const int wm = (warp & 3) * 32, wn = (warp >> 2) * 32;
   for (int s = 0; s < nsteps; ++s) {
     cp_async_wait<STAGES2 - 2>();
@@ -448,14 +484,28 @@ __global__ void __launch_bounds__(NTH, 1) dgemm2_kernel(GemmArgs g, Epi epi) {
   for (int e = threadIdx.x; e < nrl * BN; e += NTH) {
     const int r = e % nrl, c = e / nrl;
     const double* p = red + c * (BM2 + 1) + rl0 + r;
-    double v = 0.0;
-    for (int q = 0; q < splits; ++q) v += ld_cluster(p, (unsigned)q);
-    fin[c * rows + r] = v;
+    fin[c * rows + r] = sum_cluster(p, splits);
   }
   cluster_arrive();  // this CTA is done reading its peers
   __syncthreads();
   epi(m0 + rl0, min(nrl, g.Mo - (m0 + rl0)), n0, tc, fin, rows, ws);
   cluster_wait();  // peers are done reading this CTA
+}
+
+// Epilogue loop: use(e, load(e)) for this thread's elements e < n, four loads
+// in flight (the stores in between may alias them for all the compiler knows,
+// and each would wait for L2: 1 us per element of a thread, in loops of up to 16).
+template <class Load, class Use>
+__device__ __forceinline__ void each4(int n, Load load, Use use) {
+  const int bd = blockDim.x;
+  for (int e0 = threadIdx.x; e0 < n; e0 += 4 * bd) {
+    decltype(load(0)) v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = load(min(e0 + q * bd, n - 1));
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (e0 + q * bd < n) use(e0 + q * bd, v[q]);
+  }
 }
 
 // Epilogue that stores the tile: Y[r + c*ldy] for columns < W.
@@ -477,13 +527,15 @@ struct EpiStore {
 // ---------------------------------------------------------------------------
 // Largest power of two <= kMaxSplits that keeps the grid within about the
 // resident CTAs of one wave (two per SM for NT = 4, one for NT = 8) and
-// leaves every slice at least four BK steps.
+// leaves every slice a BK step: a split divides the epilogue's rows too, and at
+// small sizes that is what counts.  A 200-word, 64-column gradient of 80 products
+// took 2500 us unsplit (slices of at least four steps) and takes 605 us in eight.
 inline int pick_splits(const Context* ctx, int Mo, int Kd, int W, int NT, int tc = 0) {
   if (tc <= 0) tc = NT * 8;
   const long long tiles = (long long)((Mo + BM - 1) / BM) * ((W + tc - 1) / tc);
   const long long target = (NT <= 4 ? 2LL : 1LL) * ctx->sm_count;
   int s = 1;
-  while (s < kMaxSplits && tiles * s * 2 <= target && Kd >= s * 2 * 4 * BK) s *= 2;
+  while (s < kMaxSplits && tiles * s * 2 <= target && Kd >= s * BK) s *= 2;
   return s;
 }
 
@@ -504,13 +556,15 @@ int launch_kernel(const GemmArgs& g, const Epi& epi, cudaStream_t st) {
   cfg.blockDim = dim3(NTH);
   cfg.dynamicSmemBytes = bytes;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 1;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = (unsigned)g.splits;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   RWIG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, g, epi));
   return 0;
 }
@@ -566,13 +620,15 @@ int launch_kernel2(const GemmArgs& g, const Epi& epi, cudaStream_t st, int ntile
   cfg.blockDim = dim3(NTH);
   cfg.dynamicSmemBytes = bytes;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 1;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = (unsigned)g.splits;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   RWIG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, g, epi));
   return 0;
 }

@@ -50,7 +50,10 @@ struct Context {
   // whole-solve Sinkhorn launches (sinkhorn_resident.cu): host-mapped results
   // and the number of the last launch, which its packets' tags carry
   double* resident_res = nullptr;
-  double* range_res = nullptr;  // host-mapped: what barycenter.cu's Gibbs kernel found, for a host still enqueuing
+  // host-mapped words through which kernels of the barycenter and WDL paths
+  // tell a waiting or enqueuing host what it must know (allocated on first use)
+  static constexpr int kMappedWords = 2 + 64 * 64;
+  double* mapped = nullptr;
   unsigned long long resident_epoch = 0;
   // the K whose INT8 residue planes the scratch holds (oz::prepare_reuse):
   // its size and leading dimension, valid while no other prepare ran
@@ -84,6 +87,7 @@ bool gemm_timer_mark(Context* ctx, cudaStream_t st);
 void gemm_timer_end(Context* ctx, double* ms, int* launches);
 
 // Grow-only scratch slot `k` of at least `bytes`; nullptr on failure.
+int ensure_mapped(Context* ctx);  // Context::mapped; 0 or an engine error code
 void* scratch(Context* ctx, int k, size_t bytes);
 
 // Engine options (rwig_set_option); unknown names return `dflt`.

@@ -82,15 +82,16 @@ struct EpiY {
   double* UB;
   __device__ void operator()(int r0, int nr, int c0, int nc, double* t, int ldt, double*) const {
     if (nr <= 0) return;
-    for (int e = threadIdx.x; e < nr * nc; e += blockDim.x) {
-      const int r = e % nr, c = e / nr, gc = c0 + c;
-      if (gc >= W) continue;
-      const int i = r0 + r;
-      const size_t k = (size_t)i + (size_t)gc * N;
-      const double y = t[c * ldt + r];
-      KVB[k] = y;
-      UB[k] = A[i + (size_t)(gc % S) * N] / y;
-    }
+    dg::each4(
+        nr * nc, [&](int e) { return A[r0 + e % nr + (size_t)((c0 + e / nr) % S) * N]; },
+        [&](int e, double a) {
+          const int r = e % nr, c = e / nr, gc = c0 + c;
+          if (gc >= W) return;
+          const size_t k = (size_t)(r0 + r) + (size_t)gc * N;
+          const double y = t[c * ldt + r];
+          KVB[k] = y;
+          UB[k] = a / y;
+        });
   }
 };
 
@@ -147,12 +148,12 @@ struct EpiB1 {
     double* wg = ws + nc * ldt;  // bBbar per (group, row)
     const int ng = nc / S;
     if (!seed) {
-      for (int e = threadIdx.x; e < nr * nc; e += blockDim.x) {
-        const int r = e % nr, c = e / nr, gc = c0 + c;
-        if (gc >= W) continue;
-        const size_t k = (size_t)(r0 + r) + (size_t)gc * N;
-        ws[c * ldt + r] = (-t[c * ldt + r]) / KTU[k];  // VBbar / KTUB_l
-      }
+      dg::each4(
+          nr * nc, [&](int e) { return KTU[(size_t)(r0 + e % nr) + (size_t)min(c0 + e / nr, W - 1) * N]; },
+          [&](int e, double ktu) {
+            const int r = e % nr, c = e / nr;
+            ws[c * ldt + r] = (-t[c * ldt + r]) / ktu;  // VBbar / KTUB_l
+          });
     }
     __syncthreads();
     for (int p = threadIdx.x; p < nr * ng; p += blockDim.x) {
@@ -169,19 +170,28 @@ struct EpiB1 {
       wg[q * ldt + r] = bb;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < nr * nc; e += blockDim.x) {
-      const int r = e % nr, c = e / nr, gc = c0 + c;
-      if (gc >= W) {
-        ws[c * ldt + r] = 0.0;
-        continue;
-      }
-      const size_t k = (size_t)(r0 + r) + (size_t)gc * N;
-      const double bb = wg[(c / S) * ldt + r];
-      double tt = bb * Wb[gc];
-      if (!seed) tt -= (-t[c * ldt + r]) / KTU[k];
-      T2[k] = tt * VB[k];
-      ws[c * ldt + r] = log(KTU[k]) * (bb * bBl[(size_t)(r0 + r) + (size_t)(gc / S) * N]);
-    }
+    struct In {
+      double ktu, vb, bl, w;
+    };
+    dg::each4(
+        nr * nc,
+        [&](int e) {
+          const int r = r0 + e % nr, gc = min(c0 + e / nr, W - 1);
+          const size_t k = (size_t)r + (size_t)gc * N;
+          return In{KTU[k], VB[k], bBl[(size_t)r + (size_t)(gc / S) * N], Wb[gc]};
+        },
+        [&](int e, const In& v) {
+          const int r = e % nr, c = e / nr, gc = c0 + c;
+          if (gc >= W) {
+            ws[c * ldt + r] = 0.0;
+            return;
+          }
+          const double bb = wg[(c / S) * ldt + r];
+          double tt = bb * v.w;
+          if (!seed) tt -= (-t[c * ldt + r]) / v.ktu;
+          T2[(size_t)(r0 + r) + (size_t)gc * N] = tt * v.vb;
+          ws[c * ldt + r] = log(v.ktu) * (bb * v.bl);
+        });
     __syncthreads();
     const int n8 = (nr + 7) / 8;
     for (int p = threadIdx.x; p < n8 * nc; p += blockDim.x) {
@@ -204,14 +214,23 @@ struct EpiB2 {
   double* T;
   __device__ void operator()(int r0, int nr, int c0, int nc, double* t, int ldt, double*) const {
     if (nr <= 0) return;
-    for (int e = threadIdx.x; e < nr * nc; e += blockDim.x) {
-      const int r = e % nr, c = e / nr, gc = c0 + c;
-      if (gc >= W) continue;
-      const size_t k = (size_t)(r0 + r) + (size_t)gc * N;
-      const double y = t[c * ldt + r];
-      ABbar[k] += y / KVBprev[k];
-      T[k] = (y * UBl[k]) / KVBprev[k];
-    }
+    struct In {
+      double kv, u, ab;
+    };
+    dg::each4(
+        nr * nc,
+        [&](int e) {
+          const size_t k = (size_t)(r0 + e % nr) + (size_t)min(c0 + e / nr, W - 1) * N;
+          return In{KVBprev[k], UBl[k], ABbar[k]};
+        },
+        [&](int e, const In& v) {
+          const int r = e % nr, c = e / nr, gc = c0 + c;
+          if (gc >= W) return;
+          const size_t k = (size_t)(r0 + r) + (size_t)gc * N;
+          const double y = t[c * ldt + r];
+          ABbar[k] = v.ab + y / v.kv;
+          T[k] = (y * v.u) / v.kv;
+        });
   }
 };
 
@@ -346,8 +365,18 @@ enum {
   SW_HA, SW_HW, SW_HY, SW_HK, SW_HOUT, SW_IU, SW_IV, SW_IKV, SW_IKT, SW_IB, SW_IERR, SW_IST, SW_VCK
 };
 
-// Columns per GEMM tile: whole documents, at most 64.
-int tile_cols(int S, int SD) { return std::min((64 / S) * S, SD); }
+// Columns per GEMM tile: whole documents, at most 64.  The FP64 products take
+// tiles of at most 32, two CTAs per SM, unless those pad the columns more or the
+// 128-row tiles of the wide kernel fill the chip: 700 words, 192 columns 1982 us
+// a gradient against 2462; 1000 words with 20 topics, 960 columns, where whole
+// documents leave 12 of 32 columns empty, 12655 against 10978.
+int tile_cols(const Context* ctx, int N, int S, int SD, bool fp64) {
+  const int wide = std::min((64 / S) * S, SD);
+  if (!fp64 || S > 32) return wide;
+  const int narrow = std::min((32 / S) * S, SD);
+  const bool pads = (SD + narrow - 1) / narrow * 32 > (SD + wide - 1) / wide * 64;
+  return pads || (wide > 32 && dg::wide_tiles(N, SD, wide) >= ctx->sm_count) ? wide : narrow;
+}
 
 // ---------------------------------------------------------------------------
 // Inference (wdl_impl.cpp:349-377; cuda_wdl.cu:754-776): the parallel
@@ -373,23 +402,31 @@ struct EpiYInf {
   double* errp;
   __device__ void operator()(int r0, int nr, int c0, int nc, double* t, int ldt, double* ws) const {
     if (nr <= 0) return;
-    for (int e = threadIdx.x; e < nr * nc; e += blockDim.x) {
-      const int r = e % nr, c = e / nr, gc = c0 + c;
-      double sq = 0.0;
-      if (gc < W && active[gc / S]) {
-        const int i = r0 + r;
-        const size_t k = (size_t)i + (size_t)gc * N;
-        const double y = t[c * ldt + r];
-        const double a = A[i + (size_t)(gc % S) * N];
-        if (!first) {
-          const double res = UB[k] * y - a;
-          sq = res * res;
-        }
-        KVB[k] = y;
-        UB[k] = a / y;
-      }
-      ws[c * ldt + r] = sq;
-    }
+    struct In {
+      double a, u;
+      int on;
+    };
+    dg::each4(
+        nr * nc,
+        [&](int e) {
+          const int r = r0 + e % nr, gc = min(c0 + e / nr, W - 1);
+          return In{A[r + (size_t)(gc % S) * N], first ? 0.0 : UB[(size_t)r + (size_t)gc * N], active[gc / S]};
+        },
+        [&](int e, const In& v) {
+          const int r = e % nr, c = e / nr, gc = c0 + c;
+          double sq = 0.0;
+          if (gc < W && v.on) {
+            const size_t k = (size_t)(r0 + r) + (size_t)gc * N;
+            const double y = t[c * ldt + r];
+            if (!first) {
+              const double res = v.u * y - v.a;
+              sq = res * res;
+            }
+            KVB[k] = y;
+            UB[k] = v.a / y;
+          }
+          ws[c * ldt + r] = sq;
+        });
     if (first) return;
     __syncthreads();
     const int ng = nc / S;
@@ -445,7 +482,9 @@ struct EpiZInf {
 // document's per-row residual sums (256 strided partial sums, then a tree:
 // a fixed order), then the stopping test.  state[d] = iterations run,
 // state[D + d] = running flag, state[2 D] counts the documents still running.
-__global__ void infer_update(const double* errp, int N, int D, int L, double tol, int* state) {
+// The last document to stop stores `chunk` to host-mapped *stopped.
+__global__ void infer_update(const double* errp, int N, int D, int L, double tol, int* state, double chunk,
+                             double* stopped) {
   __shared__ double sh[256];
   const int d = blockIdx.x;
   if (!state[D + d]) return;  // the same for every thread of the block
@@ -462,7 +501,7 @@ __global__ void infer_update(const double* errp, int N, int D, int L, double tol
     const int it = ++state[d];
     if (!(it < L && err >= tol)) {
       state[D + d] = 0;
-      atomicSub(state + 2 * D, 1);
+      if (atomicSub(state + 2 * D, 1) == 1) *stopped = chunk;
     }
   }
 }
@@ -506,15 +545,19 @@ int infer(Context* ctx, cudaStream_t st, const double* A, const double* W, const
   double* errp = (double*)scratch(ctx, SW_IERR, sizeof(double) * (size_t)N * chunk);
   int* state = (int*)scratch(ctx, SW_IST, sizeof(int) * (2 * (size_t)chunk + 1));
   if (!UB || !VB || !KV || !KT || !bB || !errp || !state) return RWIG_E_NOMEM;
+  if (int rc = ensure_mapped(ctx)) return rc;
+  double* stopped = nullptr;
+  RWIG_CUDA_TRY(cudaHostGetDevicePointer((void**)&stopped, ctx->mapped, 0));
+  *ctx->mapped = 0.0;
   for (int m0 = 0; m0 < M; m0 += chunk) {
     const int D = std::min(chunk, M - m0);
     const int SD = S * D;
     const size_t NW = (size_t)N * SD;
     const double* Wb = W + (size_t)m0 * S;
-    const int tc = tile_cols(S, SD);
+    const int tc = tile_cols(ctx, N, S, SD, !pr);
     auto gemm = [&](int trans, const double* X, auto epi) -> int {
       if (pr) return oz::gemm(ctx, *pr, trans, X, N, SD, tc, epi, st, launches);
-      const dg::GemmArgs g{K, ldk, N, N, SD, X, N, 0, tc};
+      const dg::GemmArgs g{K, ldk, N, N, SD, X, N, 0, tc, 0, 1};
       return trans ? dg::gemm<1>(ctx, g, epi, st, 0, launches) : dg::gemm<0>(ctx, g, epi, st, 0, launches);
     };
     fill<<<grid_for(ctx, NW), TPB, 0, st>>>(VB, NW, 1.0);
@@ -527,13 +570,11 @@ int infer(Context* ctx, cudaStream_t st, const double* A, const double* W, const
       if (rc) return rc;
       rc = gemm(0, VB, EpiYInf{A, state + D, N, S, SD, D, 0, KV, UB, errp});
       if (rc) return rc;
-      infer_update<<<D, 256, 0, st>>>(errp, N, D, L, tol, state);
+      infer_update<<<D, 256, 0, st>>>(errp, N, D, L, tol, state, (double)(m0 + 1), stopped);
       ++*launches;
       if (tol > 0.0 && l + 1 < L) {  // stop early once every document has stopped
-        int running = 0;
-        RWIG_CUDA_TRY(cudaMemcpyAsync(&running, state + 2 * D, sizeof(int), cudaMemcpyDeviceToHost, st));
         RWIG_CUDA_TRY(cudaStreamSynchronize(st));
-        if (running == 0) break;
+        if (*ctx->mapped == (double)(m0 + 1)) break;
       }
     }
     infer_output<<<D, 1024, 0, st>>>(bB, N, Yhat + (size_t)m0 * N);
@@ -609,10 +650,10 @@ int batch_grad(Context* ctx, cudaStream_t st, double* gA, double* gl, const doub
     auto KV = [&](int t) { return KVs + NW * t + o; };
     auto KT = [&](int t) { return KTs + NW * t + o; };
     auto Bb = [&](int t) { return Bs + ND * t + od; };
-    const int tc = tile_cols(S, Wh);
+    const int tc = tile_cols(ctx, N, S, Wh, !pr);
     auto gemm = [&](int trans, const double* X, auto epi) -> int {
       if (pr) return oz::gemm(ctx, *pr, trans, X, N, Wh, tc, epi, q, launches, h);
-      const dg::GemmArgs g{K, ldk, N, N, Wh, X, N, 0, tc};
+      const dg::GemmArgs g{K, ldk, N, N, Wh, X, N, 0, tc, 0, 1};
       return trans ? dg::gemm<1>(ctx, g, epi, q, 0, launches) : dg::gemm<0>(ctx, g, epi, q, 0, launches);
     };
     const double* Wbh = Wb + c0;
