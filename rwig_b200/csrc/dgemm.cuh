@@ -288,15 +288,17 @@ __global__ void __launch_bounds__(NTH) dgemm_kernel(GemmArgs g, Epi epi) {
     cp_async_wait<STAGES - 2>();
     __syncthreads();  // stage s visible; stage s-1 no longer read
     const int nx = s + STAGES - 1;
-    if (nx < nsteps) {
-      const int q = nx % STAGES;
-      load_stage<TRANS, NT, XV>(g, As + q * ASZ, Bs + q * BSZ, m0, n0, tc, kbeg + nx * BK, kend);
-    }
-    cp_async_commit();
     const double* A = As + (s % STAGES) * ASZ;
     const double* B = Bs + (s % STAGES) * BSZ;
 #pragma unroll
     for (int k0 = 0; k0 < BK / 2; k0 += KM) {
+      if (k0 == (KM < BK / 4 ? BK / 4 : 0)) {  // while the tensor cores work on the first half of the step
+        if (nx < nsteps) {
+          const int q = nx % STAGES;
+          load_stage<TRANS, NT, XV>(g, As + q * ASZ, Bs + q * BSZ, m0, n0, tc, kbeg + nx * BK, kend);
+        }
+        cp_async_commit();
+      }
       const int kk = kh + k0;
       // A(wm + gid + 8 (i % 2), kk + tig + 4 (i / 2)), i < KM / 2
       double a[KM / 2];
