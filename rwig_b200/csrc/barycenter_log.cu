@@ -184,7 +184,9 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2) pass_kernel(Pass a) {
         }
         t = warp_sum(t);
         if (lane == 0 && s0 + q < S) {
-          part[ki * S + s0 + q] = t;
+          // a warp whose every term is exp(-inf) (zero masses, infinite costs),
+          // 0 * NaN here, adds nothing to the other warps' terms
+          part[ki * S + s0 + q] = FWD && m == -INFINITY && a.kw > 1 ? 0.0 : t;
           if (FWD) part[(a.kw + ki) * S + s0 + q] = m;
         }
       }
