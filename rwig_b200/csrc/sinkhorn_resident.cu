@@ -11,7 +11,7 @@
 // zero and drop out of every sum.  The solve is given up (status kResUnsafe,
 // and the general drivers in sinkhorn_log.cu start again from scratch) when a
 // mass is negative or not finite, when K has subnormal entries (log method), or
-// when a sum or a scaling leaves the safe range.
+// when a sum or a scaling leaves the safe range, or the gradient is not finite.
 //
 // The gradient with respect to a (Sinkhorn::_bwd_vanilla :169-213, _bwd_log
 // :379-520: one function, so one gradient) is unrolled in the same launch from
@@ -196,7 +196,7 @@ __device__ __forceinline__ void sum_block(const double* K, int lds, int nc, int 
 // Host-mapped results.
 constexpr double kResRunning = 0.0, kResFinished = 1.0, kResUnsafe = 2.0;
 enum { kResIter = 0, kResErr, kResStatus, kResLoss, kResL1Row, kResL1Col, kResL2Row, kResL2Col, kResSupM, kResSupN,
-       kResKerr, kResGradNs, kResWords };
+       kResKerr, kResGradNs, kResGradBad, kResWords };
 
 // Shared memory (doubles): block [nsm][lds], su, suo, sa [lds], sv, sd, sb
 // [ldn], colp [chunks][ldn], rowp [1024], es [8].
@@ -534,7 +534,9 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
         if (GRAD) vh[(size_t)k * ldn + tid] = v;
       }
     } else if (GRAD && stage == kBackward) {
-      if (tid < nr) sv[tid] = s * (vl * vl) * rb_j;
+      // one factor at a time: v_l^2 alone overflows from 1e154 on, v_l (K^T x)_j is
+      // of the size of the gradient's terms
+      if (tid < nr) sv[tid] = s * vl * rb_j * vl;
     }
     if (sync_or(!ok)) {
       ok = false;
@@ -649,7 +651,10 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
     errors_in();
   }
   const bool done = ok && es[1] == 1.0;
-  if (GRAD && done && ci == 0 && tid < mr) p.grad[m0 + tid] = ga;
+  if (GRAD && done && ci == 0 && tid < mr) {
+    p.grad[m0 + tid] = ga;
+    if (!isfinite(ga)) p.res[kResGradBad] = 1.0;
+  }
   if (cta == 0 && tid == 0) {
     if (GRAD && done) p.res[kResGradNs] = (double)(globaltimer_ns() - t_b);
     p.res[kResKerr] = ok && es[1] != 3.0 ? 0.0 : 1.0;
@@ -816,7 +821,7 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   p.err = (unsigned*)(info + 3);
   double* res = ctx->resident_res;
   res[kResStatus] = kResRunning;
-  res[kResKerr] = 0.0;
+  res[kResKerr] = res[kResGradBad] = 0.0;
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev0, st));
   masses_kernel<<<1, kThreads, 0, st>>>(a, b, M, N, info, p.err);
   int rc;
@@ -826,7 +831,7 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev1, st));
   RWIG_CUDA_TRY(cudaEventSynchronize(ctx->ev1));
   if (res[kResKerr] != 0.0) return set_error(RWIG_E_TIMEOUT, "Sinkhorn kernel stopped by a bounded wait");
-  if (res[kResStatus] != kResFinished) return 0;  // not in the scaling form's range
+  if (res[kResStatus] != kResFinished || res[kResGradBad] != 0.0) return 0;  // not in the scaling form's range
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   const int it = (int)res[kResIter];

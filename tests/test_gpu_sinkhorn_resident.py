@@ -86,3 +86,26 @@ def test_handed_back(reg, grad):
     assert rel_err(got["P"], ref["P"]) <= PARITY_TOL
     if grad:
         assert rel_err(got["grad_a"], ref["grad_a"]) <= PARITY_TOL
+
+
+@pytest.mark.parametrize("narrow", ["a", "b"])
+@pytest.mark.parametrize("reg", [0.002, 0.0018, 0.0016])
+@pytest.mark.parametrize("method", ["vanilla", "log"])
+def test_gradient_of_large_scalings(method, reg, narrow):
+    """Sharp kernels (max C / reg from 500 to 625) between a narrow and a broad
+    marginal: the scalings pass 1e180, their squares the range of doubles, the
+    gradient is of order one."""
+    m, n = 60, 70
+    g = synth.rng(53, m + n)
+    x = g.random((m, 1)) * (0.1 if narrow == "a" else 1.0)
+    y = g.random((n, 1)) * (1.0 if narrow == "a" else 0.1)
+    C = (x - y.T) ** 2
+    C /= C.max()
+    a, b = synth.dirichlet(g, 1.0, m), synth.dirichlet(g, 1.0, n)
+    got = rw.sinkhorn(a, b, C, {"reg": reg, "method": method, "with_grad": True, "max_iter": 10, "zero_tol": 0.0})
+    assert rw.last_report()["kernel_launches"] == RESIDENT_LAUNCHES
+    if method == "vanilla":
+        assert max(got["u"].max(), got["v"].max()) > 1e155
+    ref = ORACLE[method](a, b, C, reg, with_grad=True, max_iter=10, zero_tol=0.0)
+    assert np.isfinite(ref["grad_a"]).all()
+    _same(got, ref, reg, method)
