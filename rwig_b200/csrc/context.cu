@@ -173,6 +173,14 @@ void* scratch(Context* ctx, int k, size_t bytes) {
   return p;
 }
 
+int raise_smem(Context* ctx, const void* kern, size_t bytes) {
+  size_t& have = ctx->smem_raised[kern];
+  if (have >= bytes) return 0;
+  RWIG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  have = bytes;
+  return 0;
+}
+
 int ensure_mapped(Context* ctx) {
   if (!ctx->mapped)
     RWIG_CUDA_TRY(cudaHostAlloc((void**)&ctx->mapped, sizeof(double) * Context::kMappedWords, cudaHostAllocMapped));

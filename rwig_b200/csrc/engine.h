@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -55,6 +56,8 @@ struct Context {
   static constexpr int kMappedWords = 2 + 64 * 64;
   double* mapped = nullptr;
   unsigned long long resident_epoch = 0;
+  // dynamic shared memory each kernel may use on this device (raise_smem)
+  std::map<const void*, size_t> smem_raised;
   // the K whose INT8 residue planes the scratch holds (oz::prepare_reuse):
   // its size and leading dimension, valid while no other prepare ran
   bool oz_kept = false;
@@ -85,6 +88,11 @@ cudaStream_t side_stream(Context* ctx, int i);
 int gemm_timer_begin(Context* ctx);
 bool gemm_timer_mark(Context* ctx, cudaStream_t st);
 void gemm_timer_end(Context* ctx, double* ms, int* launches);
+
+// Lets `kern` use `bytes` of dynamic shared memory on the context's device, which
+// is current; 0 or an engine error code.  The limit belongs to a kernel on one
+// device: a process that uses several raises it on each.
+int raise_smem(Context* ctx, const void* kern, size_t bytes);
 
 // Grow-only scratch slot `k` of at least `bytes`; nullptr on failure.
 int ensure_mapped(Context* ctx);  // Context::mapped; 0 or an engine error code

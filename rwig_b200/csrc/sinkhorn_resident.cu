@@ -743,13 +743,9 @@ bool shape(const Context* ctx, int M, int N, Shape* best) {
 }
 
 template <bool GRAD, bool REG>
-int launch(Args& p, const Shape& s, cudaStream_t st) {
+int launch(Context* ctx, Args& p, const Shape& s, cudaStream_t st) {
   auto kern = resident_kernel<GRAD, REG>;
-  static size_t attr = 0;  // callers hold the context lock
-  if (attr < s.smem) {
-    RWIG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem));
-    attr = s.smem;
-  }
+  if (int rc = raise_smem(ctx, (const void*)kern, s.smem)) return rc;
   void* args[] = {&p};
   RWIG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)kern, dim3(s.gr * s.gc), dim3(kThreads), args, s.smem, st));
   return 0;
@@ -825,8 +821,8 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev0, st));
   masses_kernel<<<1, kThreads, 0, st>>>(a, b, M, N, info, p.err);
   int rc;
-  if (grad) rc = s.reg ? launch<true, true>(p, s, st) : launch<true, false>(p, s, st);
-  else rc = s.reg ? launch<false, true>(p, s, st) : launch<false, false>(p, s, st);
+  if (grad) rc = s.reg ? launch<true, true>(ctx, p, s, st) : launch<true, false>(ctx, p, s, st);
+  else rc = s.reg ? launch<false, true>(ctx, p, s, st) : launch<false, false>(ctx, p, s, st);
   if (rc) return rc;
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev1, st));
   RWIG_CUDA_TRY(cudaEventSynchronize(ctx->ev1));
