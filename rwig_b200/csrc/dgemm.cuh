@@ -544,14 +544,10 @@ inline int pick_splits(const Context* ctx, int Mo, int Kd, int W, int NT, int tc
 inline int clamp_splits(int s) { return s >= 8 ? 8 : s >= 4 ? 4 : s >= 2 ? 2 : 1; }
 
 template <int TRANS, int NT, int XV, class Epi, int KM>
-int launch_kernel(const GemmArgs& g, const Epi& epi, cudaStream_t st) {
+int launch_kernel(Context* ctx, const GemmArgs& g, const Epi& epi, cudaStream_t st) {
   constexpr size_t bytes = sizeof(double) * smem_doubles<TRANS, NT>();
   auto kern = dgemm_kernel<TRANS, NT, XV, Epi, KM>;
-  static bool attr_set = false;  // once per instantiation (callers hold the context lock)
-  if (!attr_set) {
-    RWIG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    attr_set = true;
-  }
+  if (int rc = raise_smem(ctx, (const void*)kern, bytes)) return rc;
   cudaLaunchConfig_t cfg = {};
   const int tc = g.tcols > 0 ? g.tcols : NT * 8;
   cfg.gridDim = dim3((unsigned)(((g.Mo + BM - 1) / BM) * ((g.W + tc - 1) / tc)), 1, g.splits);
@@ -572,25 +568,20 @@ int launch_kernel(const GemmArgs& g, const Epi& epi, cudaStream_t st) {
 }
 
 template <int TRANS, int XV, class Epi, int KM>
-int prepare_kernel2() {
+int prepare_kernel2(Context* ctx) {
   constexpr size_t bytes = sizeof(double) * smem2_doubles<TRANS>();
   static_assert(bytes <= 227 * 1024, "wide-tile GEMM exceeds the shared memory of a CTA");
-  static bool attr_set = false;  // once per instantiation (callers hold the context lock)
-  if (!attr_set) {
-    RWIG_CUDA_TRY(cudaFuncSetAttribute(dgemm2_kernel<TRANS, XV, Epi, KM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)bytes));
-    attr_set = true;
-  }
-  return 0;
+  return raise_smem(ctx, (const void*)dgemm2_kernel<TRANS, XV, Epi, KM>, bytes);
 }
 
 // Clusters of `s` wide-tile CTAs that can be resident at once (cached per
-// instantiation; 0 if the query fails).
+// device and instantiation; 0 if the query fails).
 template <int TRANS, int XV, class Epi, int KM>
-int max_clusters2(int s) {
-  static int cache[kMaxSplits + 1] = {};
+int max_clusters2(Context* ctx, int s) {
+  static_assert(kMaxSplits < Context::kClusterSizes, "cluster sizes of the cache");
+  int* const cache = ctx->clusters[(const void*)dgemm2_kernel<TRANS, XV, Epi, KM>].data();
   if (cache[s] == 0) {
-    if (prepare_kernel2<TRANS, XV, Epi, KM>() != 0) return 0;
+    if (prepare_kernel2<TRANS, XV, Epi, KM>(ctx) != 0) return 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1, 1, (unsigned)s);
     cfg.blockDim = dim3(NTH);
@@ -613,10 +604,10 @@ int max_clusters2(int s) {
 }
 
 template <int TRANS, int XV, class Epi, int KM>
-int launch_kernel2(const GemmArgs& g, const Epi& epi, cudaStream_t st, int ntile) {
+int launch_kernel2(Context* ctx, const GemmArgs& g, const Epi& epi, cudaStream_t st, int ntile) {
   constexpr size_t bytes = sizeof(double) * smem2_doubles<TRANS>();
   auto kern = dgemm2_kernel<TRANS, XV, Epi, KM>;
-  if (int rc = prepare_kernel2<TRANS, XV, Epi, KM>()) return rc;
+  if (int rc = prepare_kernel2<TRANS, XV, Epi, KM>(ctx)) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ntile, 1, g.splits);
   cfg.blockDim = dim3(NTH);
@@ -656,21 +647,21 @@ inline long long wide_tiles(int Mo, int W, int tc) {
 // partial wave (when they fill at most half the SMs) as a second launch with
 // split-K, so the tail takes a fraction of a wave.
 template <int TRANS, int XV, class Epi, int KM>
-int gemm_wide(const Context* ctx, GemmArgs g, const Epi& epi, cudaStream_t st, int* launches) {
+int gemm_wide(Context* ctx, GemmArgs g, const Epi& epi, cudaStream_t st, int* launches) {
   const long long tiles = wide_tiles(g.Mo, g.W, g.tcols);
   const int sm = ctx->sm_count;
   if (g.splits > 0 || tiles < sm) {
     g.splits = g.splits > 0 ? std::min(g.splits, kMaxSplits) : pick_splits2(ctx, tiles, g.Kd);
     g.tile0 = 0;
     if (launches) ++*launches;
-    return launch_kernel2<TRANS, XV, Epi, KM>(g, epi, st, (int)tiles);
+    return launch_kernel2<TRANS, XV, Epi, KM>(ctx, g, epi, st, (int)tiles);
   }
   const long long tail = tiles % sm;
   const long long full = (tail > 0 && 2 * tail <= sm) ? tiles - tail : tiles;
   g.splits = 1;
   g.tile0 = 0;
   if (launches) ++*launches;
-  int rc = launch_kernel2<TRANS, XV, Epi, KM>(g, epi, st, (int)full);
+  int rc = launch_kernel2<TRANS, XV, Epi, KM>(ctx, g, epi, st, (int)full);
   if (rc != 0 || full == tiles) return rc;
   // split count of the tail: the least waves of resident clusters per slice,
   // ceil(tail / clusters(s)) / s (clusters wider than a TPC pair may leave SMs
@@ -678,7 +669,7 @@ int gemm_wide(const Context* ctx, GemmArgs g, const Epi& epi, cudaStream_t st, i
   int best = 1;
   double best_t = 1.0;
   for (int s = 2; s <= kMaxSplits && g.Kd >= s * 4 * BK; ++s) {
-    const int nc = max_clusters2<TRANS, XV, Epi, KM>(s);
+    const int nc = max_clusters2<TRANS, XV, Epi, KM>(ctx, s);
     if (nc < 1) continue;
     const double t = (double)((tail + nc - 1) / nc) / s;
     if (t < best_t - 1e-9) {
@@ -689,7 +680,7 @@ int gemm_wide(const Context* ctx, GemmArgs g, const Epi& epi, cudaStream_t st, i
   g.splits = best;
   g.tile0 = (int)full;
   if (launches) ++*launches;
-  return launch_kernel2<TRANS, XV, Epi, KM>(g, epi, st, (int)(tiles - full));
+  return launch_kernel2<TRANS, XV, Epi, KM>(ctx, g, epi, st, (int)(tiles - full));
 }
 
 // tile: 0 picks the tile height (128 rows for tiles of more than 32 columns
@@ -698,7 +689,7 @@ int gemm_wide(const Context* ctx, GemmArgs g, const Epi& epi, cudaStream_t st, i
 // incremented by the number of kernel launches made (1, or 2 with a split
 // tail wave).
 template <int TRANS, class Epi, int KM = kDmmaK>
-int gemm(const Context* ctx, GemmArgs g, const Epi& epi, cudaStream_t st, int tile = 0, int* launches = nullptr) {
+int gemm(Context* ctx, GemmArgs g, const Epi& epi, cudaStream_t st, int tile = 0, int* launches = nullptr) {
   if (!g.K || !g.X || g.Mo < 1 || g.Kd < 1 || g.W < 1)
     return set_error(RWIG_E_INVALID, "GEMM: null operand or empty shape");
   if ((g.ldk % 2) != 0 || (reinterpret_cast<uintptr_t>(g.K) % 16) != 0)
@@ -718,8 +709,10 @@ int gemm(const Context* ctx, GemmArgs g, const Epi& epi, cudaStream_t st, int ti
   g.splits = g.splits <= 0 ? pick_splits(ctx, g.Mo, g.Kd, g.W, NT, g.tcols) : clamp_splits(g.splits);
   if (launches) ++*launches;
   if (NT == 4)
-    return xv2 ? launch_kernel<TRANS, 4, 2, Epi, KM>(g, epi, st) : launch_kernel<TRANS, 4, 1, Epi, KM>(g, epi, st);
-  return xv2 ? launch_kernel<TRANS, 8, 2, Epi, KM>(g, epi, st) : launch_kernel<TRANS, 8, 1, Epi, KM>(g, epi, st);
+    return xv2 ? launch_kernel<TRANS, 4, 2, Epi, KM>(ctx, g, epi, st)
+               : launch_kernel<TRANS, 4, 1, Epi, KM>(ctx, g, epi, st);
+  return xv2 ? launch_kernel<TRANS, 8, 2, Epi, KM>(ctx, g, epi, st)
+             : launch_kernel<TRANS, 8, 1, Epi, KM>(ctx, g, epi, st);
 }
 
 }  // namespace dg

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstddef>
 #include <map>
 #include <mutex>
@@ -58,6 +59,10 @@ struct Context {
   unsigned long long resident_epoch = 0;
   // dynamic shared memory each kernel may use on this device (raise_smem)
   std::map<const void*, size_t> smem_raised;
+  // clusters of each size that can be resident at once, by kernel (dgemm.cuh; 0
+  // not asked, -1 none)
+  static constexpr int kClusterSizes = 9;
+  std::map<const void*, std::array<int, kClusterSizes>> clusters;
   // the K whose INT8 residue planes the scratch holds (oz::prepare_reuse):
   // its size and leading dimension, valid while no other prepare ran
   bool oz_kept = false;

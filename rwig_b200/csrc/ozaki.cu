@@ -551,17 +551,14 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  static const EncodeTiledFn fn = []() -> EncodeTiledFn {  // (once, whichever device's thread comes first)
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q{};
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
+    const bool found = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess;
     (void)cudaGetLastError();
-  }
+    return found ? reinterpret_cast<EncodeTiledFn>(p) : nullptr;
+  }();
   return fn;
 }
 
@@ -615,21 +612,14 @@ int launch_i8(Context* ctx, const int8_t* A, int Mpad, const int8_t* B, int Wpad
   const int MT = tm_opt == 128 || tm_opt == 256 ? tm_opt : 256;
   if (int rc = make_map(&ta, A, Kpad, Mpad, planes, MT)) return rc;
   if (int rc = make_map(&tb, B, Kpad, Wpad, planes, ntile)) return rc;
-  static bool attr[2] = {false, false};
   const int ntn = Wpad / ntile, ntm = Mpad / MT, tiles = ntn * ntm * planes;
   const int grid = std::min(tiles, ctx->sm_count);  // persistent: one CTA per SM
   const bool timed = gemm_timer_mark(ctx, st);
   if (MT == 256) {
-    if (!attr[0]) {
-      RWIG_CUDA_TRY(cudaFuncSetAttribute(i8_gemm<RAW, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
-      attr[0] = true;
-    }
+    if (int rc = raise_smem(ctx, (const void*)i8_gemm<RAW, 256>, kGemmSmem)) return rc;
     i8_gemm<RAW, 256><<<grid, kPersistThreads, kGemmSmem, st>>>(ta, tb, g, ntn, ntm, planes);
   } else {
-    if (!attr[1]) {
-      RWIG_CUDA_TRY(cudaFuncSetAttribute(i8_gemm<RAW, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
-      attr[1] = true;
-    }
+    if (int rc = raise_smem(ctx, (const void*)i8_gemm<RAW, 128>, kGemmSmem)) return rc;
     i8_gemm<RAW, 128><<<grid, kPersistThreads, kGemmSmem, st>>>(ta, tb, g, ntn, ntm, planes);
   }
   RWIG_CUDA_TRY(cudaGetLastError());

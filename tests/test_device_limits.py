@@ -23,9 +23,9 @@ def test_shared_memory_limit_is_raised_on_each_device(tmp_path):
     assert run.returncode == 0, run.stdout
 
 
-@pytest.mark.parametrize("name", ["sinkhorn_resident.cu"])
+@pytest.mark.parametrize("name", ["sinkhorn_resident.cu", "dgemm.cuh", "ozaki.cu", "ozaki.cuh", "batch.cu"])
 def test_no_process_wide_guard(name):
     """No static variable guards a cudaFuncSetAttribute call."""
     src = open(os.path.join(CSRC, name)).read()
-    assert not re.search(r"\bstatic (bool|int|size_t) attr", src)
+    assert not re.search(r"\bstatic (bool|int|size_t) (attr|cache|tried)", src)
     assert "raise_smem(" in src
