@@ -49,6 +49,7 @@
 
 #include "common.cuh"
 #include "engine.h"
+#include "resident_words.h"
 #include "sk_host.h"
 
 namespace rwig {
@@ -192,11 +193,6 @@ __device__ __forceinline__ void sum_block(const double* K, int lds, int nc, int 
     if (rl == 0 && c < nc) out[c] = t;
   }
 }
-
-// Host-mapped results.
-constexpr double kResRunning = 0.0, kResFinished = 1.0, kResUnsafe = 2.0;
-enum { kResIter = 0, kResErr, kResStatus, kResLoss, kResL1Row, kResL1Col, kResL2Row, kResL2Col, kResSupM, kResSupN,
-       kResKerr, kResGradNs, kResGradBad, kResWords };
 
 // Shared memory (doubles): block [nsm][lds], su, suo, sa [lds], sv, sd, sb
 // [ldn], colp [chunks][ldn], rowp [1024], es [8].
@@ -655,10 +651,9 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
     p.grad[m0 + tid] = ga;
     if (!isfinite(ga)) p.res[kResGradBad] = 1.0;
   }
-  if (cta == 0 && tid == 0) {
-    if (GRAD && done) p.res[kResGradNs] = (double)(globaltimer_ns() - t_b);
-    p.res[kResKerr] = ok && es[1] != 3.0 ? 0.0 : 1.0;
-    p.res[kResStatus] = done ? kResFinished : kResUnsafe;
+  if (tid == 0) {
+    if (GRAD && done && cta == 0) p.res[kResGradNs] = (double)(globaltimer_ns() - t_b);
+    words_leave(p.res, cta, ok && es[1] != 3.0, done);
   }
 }
 
@@ -816,8 +811,7 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   p.res = dres;
   p.err = (unsigned*)(info + 3);
   double* res = ctx->resident_res;
-  res[kResStatus] = kResRunning;
-  res[kResKerr] = res[kResGradBad] = 0.0;
+  words_clear(res);
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev0, st));
   masses_kernel<<<1, kThreads, 0, st>>>(a, b, M, N, info, p.err);
   int rc;
@@ -826,8 +820,9 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   if (rc) return rc;
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev1, st));
   RWIG_CUDA_TRY(cudaEventSynchronize(ctx->ev1));
-  if (res[kResKerr] != 0.0) return set_error(RWIG_E_TIMEOUT, "Sinkhorn kernel stopped by a bounded wait");
-  if (res[kResStatus] != kResFinished || res[kResGradBad] != 0.0) return 0;  // not in the scaling form's range
+  const int outcome = words_outcome(res);
+  if (outcome < 0) return set_error(RWIG_E_TIMEOUT, "Sinkhorn kernel stopped by a bounded wait");
+  if (outcome == 0) return 0;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   const int it = (int)res[kResIter];
