@@ -147,8 +147,9 @@ RWIG_API int rwig_get_option(const char* name, double* value);
  * may be NULL): P (M x N), grad_a (M, needs withgrad), u (M), v (N), loss.
  * grad_a is the unrolled backward Sinkhorn::_bwd_vanilla (:169-213), zero off
  * the support; it needs at most 8192 non-zero entries of a and keeps every
- * iteration's scalings on the device (8 (max_iter + 2)(M + N) bytes, at most
- * 32 GiB), else RWIG_E_UNSUPPORTED.
+ * iteration's scalings on the device (8 (max_iter + 4)(M + N) bytes, in scratch
+ * kept until rwig_shutdown; more than 32 GiB, counted over the support and
+ * max_iter + 2, is RWIG_E_UNSUPPORTED).
  */
 RWIG_API int rwig_sinkhorn_vanilla(double* P, double* grad_a, double* u, double* v, double* loss,
                                    int* iter, double* err, const double* a, const double* b,

@@ -703,9 +703,7 @@ enum {
   SL_CTRL, SL_RES, SL_CRED, SL_AR, SL_BR, SL_RIDX, SL_CIDX, SL_HOST_C, SL_HOST_A, SL_HOST_B,
   SL_HOST_P, SL_HOST_F, SL_HOST_G, SL_FST, SL_GST, SL_FT, SL_GT, SL_KT, SL_U0, SL_U1, SL_FH, SL_GH, SL_HOST_GA
 };
-
-// Largest forward history kept for the gradient (f and g of every iteration).
-constexpr size_t kMaxHistoryBytes = size_t(32) << 30;
+static_assert(SL_FH == kSlotHistoryF && SL_GH == kSlotHistoryG, "history slots");
 
 // Core of both log-Sinkhorn entry points: inputs on the device.
 __global__ void scatter_kernel(const double* x, const int* idx, int n, double* out) {

@@ -95,11 +95,10 @@ struct Args {
   double* f;        // optional: f / u
   double* g;        // optional: g / v
   double* grad;     // gradient: M
-  double* uh;       // gradient: u_l of each CTA's rows at [cta][l][ldm]
-  double* vh;       // gradient: v_l of each CTA's columns at [cta][l][ldn]
+  double* uh;       // gradient: u_l at [l][M], stored by the first CTA of each block row
+  double* vh;       // gradient: v_l at [l][N], stored by the first CTA of each block column
   const double* info;  // masses_kernel: support sizes, bad masses
-  int M, N, gr, gc, lds, ldm, ldn, nsm, chunks;
-  int vanilla, max_iter;
+  int M, N, gr, gc, lds, vanilla, ldn, nsm, chunks, max_iter;
   double eps, tol;
   // packets, two exchanges of each kind by the tag's parity: a CTA may send the
   // next one's while a peer still reads this one's, but not the one after that,
@@ -404,8 +403,8 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
     return t;
   };
   auto in_range = [](double x) { return x >= kLo && x <= kHi; };
-  double* const uh = GRAD ? p.uh + (size_t)cta * (p.max_iter + 4) * p.ldm : nullptr;
-  double* const vh = GRAD ? p.vh + (size_t)cta * (p.max_iter + 4) * ldn : nullptr;
+  double* const uh = GRAD ? p.uh + m0 : nullptr;
+  double* const vh = GRAD ? p.vh + n0 : nullptr;
   // Packets of exchange e: each CTA's shares of the row and the column error.
   auto error_at = [&](unsigned long long e) { return p.epart + (e & 3) * 2 * G; };
 
@@ -508,6 +507,10 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
         fi = eps * log(u);
         const double gj = eps * log(v);
         if (es[1] != 1.0) break;
+        // the histories, stored by one CTA of each block row and column, are out
+        // before this thread's next packets, which the same thread of every
+        // other CTA there waits for (in kMargins) before it reads them
+        if (GRAD) __threadfence();
         sync();
         if (tid < mr) {
           su[tid] = fi;
@@ -527,7 +530,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
         sv[tid] = v;
         const double d = p.vanilla ? fma(v, s, -b_j) : fma(v, s, -b_j) * rb_j;  // log(v s / b) to first order
         sd[tid] = b_j == 0.0 ? 0.0 : in_range(s) && in_range(v) ? d * d : INFINITY;
-        if (GRAD) vh[(size_t)k * ldn + tid] = v;
+        if (GRAD && ri == 0) vh[(size_t)k * N + tid] = v;
       }
     } else if (GRAD && stage == kBackward) {
       // one factor at a time: v_l^2 alone overflows from 1e154 on, v_l (K^T x)_j is
@@ -550,7 +553,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
       if (tid < mr) {
         suo[tid] = u1;
         su[tid] = u;
-        if (GRAD) uh[(size_t)k * p.ldm + tid] = u;
+        if (GRAD && ci == 0) uh[(size_t)k * M + tid] = u;
       }
       if (sync_or(!ok)) {
         ok = false;
@@ -599,6 +602,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
         }
       }
       if (!GRAD) break;
+      __threadfence();  // (after the packets of the CTAs that stored the histories)
       t_b = globaltimer_ns();
       // a plan entry that underflowed: the reference's sums turn NaN or infinite
       // there, which the general path reproduces
@@ -632,8 +636,9 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
       --l;
       if (l == 0) break;
       if (tid < mr) su[tid] = q * ul;
-      ul = tid < mr && a_i != 0.0 ? uh[(size_t)l * p.ldm + tid] : 0.0;  // (written by this thread)
-      vl = tid < nr ? vh[(size_t)l * ldn + tid] : 0.0;
+      // (from L2: plain loads of lines that other CTAs share cost 0.8% of a call)
+      ul = tid < mr && a_i != 0.0 ? __ldcg(uh + (size_t)l * M + tid) : 0.0;
+      vl = tid < nr ? __ldcg(vh + (size_t)l * N + tid) : 0.0;
       stage = kBackward;
       if (sync_or(!ok)) {
         ok = false;
@@ -746,7 +751,7 @@ int launch(Context* ctx, Args& p, const Shape& s, cudaStream_t st) {
   return 0;
 }
 
-enum { SRS_PACKETS = 250, SRS_INFO, SRS_UH, SRS_VH };
+enum { SRS_PACKETS = 250, SRS_INFO };
 
 }  // namespace skres
 
@@ -758,10 +763,10 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   Shape s;
   if (max_iter < 1 || !(zero_tol <= 999.0) || !shape(ctx, M, N, &s)) return 0;
   const size_t G = (size_t)s.gr * s.gc, L2 = (size_t)max_iter + 4;
-  // each CTA keeps its own scalings of every iteration, which takes gr + gc
-  // times the general drivers' history: at most 4 GB of it (2048^2: max_iter
-  // 10000), and the general drivers when it cannot be had
-  if (grad && 8 * L2 * G * (s.ldm + s.ldn) > (size_t(4) << 30)) return 0;
+  // the scalings of every iteration, in the general drivers' own slots: they are
+  // of the same size, so what cannot be had here is refused there
+  const size_t bytes_u = 8 * L2 * (size_t)M, bytes_v = 8 * L2 * (size_t)N;
+  if (grad && bytes_u + bytes_v > kMaxHistoryBytes) return 0;
   if (!ctx->resident_res) {
     void* h = nullptr;
     RWIG_CUDA_TRY(cudaHostAlloc(&h, sizeof(double) * kResWords, cudaHostAllocMapped));
@@ -774,8 +779,8 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   const bool fresh = (int)ctx->slots.size() <= SRS_PACKETS || ctx->slot_bytes[SRS_PACKETS] < bytes;
   Packet* pk = (Packet*)scratch(ctx, SRS_PACKETS, bytes);
   double* info = (double*)scratch(ctx, SRS_INFO, sizeof(double) * 4);
-  double* uh = grad ? (double*)scratch(ctx, SRS_UH, 8 * L2 * G * s.ldm) : nullptr;
-  double* vh = grad ? (double*)scratch(ctx, SRS_VH, 8 * L2 * G * s.ldn) : nullptr;
+  double* uh = grad ? (double*)scratch(ctx, kSlotHistoryF, bytes_u) : nullptr;
+  double* vh = grad ? (double*)scratch(ctx, kSlotHistoryG, bytes_v) : nullptr;
   if (!pk || !info || (grad && (!uh || !vh))) return 0;
   if (fresh)  // no packet of an earlier life of this memory may carry a tag to come
     RWIG_CUDA_TRY(cudaMemsetAsync(pk, 0, ctx->slot_bytes[SRS_PACKETS], st));
@@ -795,7 +800,6 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   p.gr = s.gr;
   p.gc = s.gc;
   p.lds = s.lds;
-  p.ldm = s.ldm;
   p.ldn = s.ldn;
   p.nsm = s.nsm;
   p.chunks = s.chunks;

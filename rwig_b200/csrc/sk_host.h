@@ -57,6 +57,11 @@ int sinkhorn_grad(Context* ctx, cudaStream_t st, bool vanilla, const double* C, 
                   const double* gh, int m, int n, int L, double eps, const int* ridx, int M, double out_scale,
                   double* grad_a, int* launches);
 
+// Scratch slots of a gradient's history (f or u, g or v of every iteration),
+// shared by the drivers of one context, and the largest history kept.
+constexpr int kSlotHistoryF = 31, kSlotHistoryG = 32;
+constexpr size_t kMaxHistoryBytes = size_t(32) << 30;
+
 // A whole solve in one launch (sinkhorn_resident.cu), grad_a optional: 1 with
 // *status and the report filled, 0 when the problem does not fit or left the
 // scaling form's range (nothing of its outputs is to be used), < 0 an error.

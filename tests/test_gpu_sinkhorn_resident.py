@@ -109,3 +109,25 @@ def test_gradient_of_large_scalings(method, reg, narrow):
     ref = ORACLE[method](a, b, C, reg, with_grad=True, max_iter=10, zero_tol=0.0)
     assert np.isfinite(ref["grad_a"]).all()
     _same(got, ref, reg, method)
+
+
+def test_gradient_history_memory():
+    """A gradient keeps each iteration's scalings once, not once per block:
+    8 (max_iter + 4)(M + N) bytes, sized by max_iter."""
+    import torch
+    m, n, max_iter = 600, 500, 5000
+    a, b, C = _problem(m, n)
+    rw.load().rwig_shutdown()  # start without scratch
+
+    def solve(iters):
+        before = torch.cuda.mem_get_info()[0]
+        r = rw.sinkhorn(a, b, C, {"reg": 0.2, "method": "log", "with_grad": True, "max_iter": iters})
+        assert rw.last_report()["kernel_launches"] == RESIDENT_LAUNCHES and r["iter"] < 100
+        return before - torch.cuda.mem_get_info()[0], r
+
+    torch.cuda.mem_get_info()
+    _, ref = solve(100)  # the context, module and all other scratch
+    grown, got = solve(max_iter)
+    # allocations are rounded to 2 MB blocks
+    assert grown <= 8 * (max_iter + 4) * (m + n) + 2 * (2 << 20)
+    assert np.array_equal(got["grad_a"], ref["grad_a"])
