@@ -53,7 +53,9 @@ typedef struct rwig_report {
   double sweep_ms;       /* device time of the launches that ran scaled-form iterations */
   int sweep_iters;       /* iterations run by those launches */
   int fallback_events;   /* sweeps re-run with exact per-row / per-column minima
-                            (log barycenter: 1 when the log-domain kernels ran) */
+                            (log barycenter: 1 when the log-domain kernels ran;
+                            Sinkhorn: one more when a solve in one launch left
+                            the scaling form's range and was started again) */
   int kernel_launches;   /* engine kernels launched by the call */
   int support_m;         /* rows kept after dropping zero-mass entries of a */
   int support_n;         /* columns kept after dropping zero-mass entries of b */

@@ -729,14 +729,15 @@ int sinkhorn_device(Context* ctx, cudaStream_t st, bool vanilla, double* P, doub
   // Problems that fit on the chip run in one launch.  The log method asks for
   // the scaling form with its default absorption bound; a problem that leaves
   // the form's range comes back here and starts again.
+  int launches = 0;  // those of a solve that comes back count
   if (vanilla || (option("log_sinkhorn.scaled", 1.0) != 0.0 && option("log_sinkhorn.tau", 100.0) >= 100.0)) {
     int status = 0;
     const int rc = sinkhorn_resident(ctx, st, vanilla, P, want_grad ? grad_a : nullptr, f, g, loss, iter, err, a, b, C,
-                                     M, N, reg, max_iter, zero_tol, &status);
+                                     M, N, reg, max_iter, zero_tol, &status, &launches);
     if (rc < 0) return rc;
     if (rc > 0) return status;
   }
-  int launches = 0;
+  const bool handed_back = launches > 0;
 
   // support reduction (src/sinkhorn_impl_log.cpp:238-249): drop zero masses
   std::vector<double> ha(M), hb(N);
@@ -758,7 +759,7 @@ int sinkhorn_device(Context* ctx, cudaStream_t st, bool vanilla, double* P, doub
   const bool need_gather = reduced || (M % 2) != 0 || (reinterpret_cast<uintptr_t>(C) % 16) != 0;
   const long long ldc = need_gather ? ((m + 1) / 2) * 2 : M;
 
-  RWIG_CUDA_TRY(cudaEventRecord(ctx->ev0, st));
+  if (!handed_back) RWIG_CUDA_TRY(cudaEventRecord(ctx->ev0, st));  // (else recorded before the resident launches)
   int* d_ridx = nullptr;
   int* d_cidx = nullptr;
   const double* Cr = C;
@@ -864,7 +865,7 @@ int sinkhorn_device(Context* ctx, cudaStream_t st, bool vanilla, double* P, doub
 
   double res[16];
   unsigned ctrl[4];
-  int fallbacks = 0;
+  int fallbacks = handed_back ? 1 : 0;
   double sweep_ms = 0.0;
   int sweep_iters = 0;
   // Runs one cooperative launch of `launch_fn` and reads back its results.

@@ -757,7 +757,7 @@ enum { SRS_PACKETS = 250, SRS_INFO };
 
 int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, double* grad_a, double* f, double* g,
                       double* loss, int* iter, double* err, const double* a, const double* b, const double* C, int M,
-                      int N, double reg, int max_iter, double zero_tol, int* status_out) {
+                      int N, double reg, int max_iter, double zero_tol, int* status_out, int* launches) {
   using namespace skres;
   const bool grad = grad_a != nullptr;
   Shape s;
@@ -822,6 +822,7 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   if (grad) rc = s.reg ? launch<true, true>(ctx, p, s, st) : launch<true, false>(ctx, p, s, st);
   else rc = s.reg ? launch<false, true>(ctx, p, s, st) : launch<false, false>(ctx, p, s, st);
   if (rc) return rc;
+  *launches = 2;
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev1, st));
   RWIG_CUDA_TRY(cudaEventSynchronize(ctx->ev1));
   const int outcome = words_outcome(res);
@@ -848,7 +849,7 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   R.grad_ms = res[kResGradNs] * 1e-6;
   R.sweep_ms = ms - R.grad_ms;
   R.sweep_iters = it;
-  R.kernel_launches = 2;
+  R.kernel_launches = *launches;
   R.support_m = (int)res[kResSupM];
   R.support_n = (int)res[kResSupN];
   return 1;

@@ -64,10 +64,11 @@ constexpr size_t kMaxHistoryBytes = size_t(32) << 30;
 
 // A whole solve in one launch (sinkhorn_resident.cu), grad_a optional: 1 with
 // *status and the report filled, 0 when the problem does not fit or left the
-// scaling form's range (nothing of its outputs is to be used), < 0 an error.
+// scaling form's range (nothing of its outputs is to be used; *launches counts
+// what ran from event ev0 on, none when it does not fit), < 0 an error.
 int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, double* grad_a, double* f, double* g,
                       double* loss, int* iter, double* err, const double* a, const double* b, const double* C, int M,
-                      int N, double reg, int max_iter, double zero_tol, int* status);
+                      int N, double reg, int max_iter, double zero_tol, int* status, int* launches);
 
 int sinkhorn_device(Context* ctx, cudaStream_t st, bool vanilla, double* P, double* grad_a, double* f, double* g,
                     double* loss, int* iter, double* err, const double* a, const double* b, const double* C,

@@ -131,3 +131,30 @@ def test_gradient_history_memory():
     # allocations are rounded to 2 MB blocks
     assert grown <= 8 * (max_iter + 4) * (m + n) + 2 * (2 << 20)
     assert np.array_equal(got["grad_a"], ref["grad_a"])
+
+
+@pytest.mark.parametrize("method", ["vanilla", "log"])
+def test_report_of_a_handed_back_call(method):
+    """The launches and the time of a solve in one launch that was given up are
+    in the report: two launches more than the general drivers alone take."""
+    a, b, C = _problem(90, 70)
+    a[0] = 1e-280  # its scaling leaves the safe range
+    par = {"reg": 0.1, "method": method, "max_iter": 12, "zero_tol": 0.0}
+    L = rw.load()
+    got = rw.sinkhorn(a, b, C, par)
+    back = rw.last_report()
+    assert back["iter"] == got["iter"] == 12
+    assert back["device_ms"] > back["kernel_ms"]
+    if method == "log":
+        L.rwig_set_option(b"log_sinkhorn.tau", 99.0)
+        try:
+            ref = rw.sinkhorn(a, b, C, par)
+        finally:
+            L.rwig_set_option(b"log_sinkhorn.tau", float("nan"))
+        general = rw.last_report()
+        assert back["fallback_events"] == general["fallback_events"] + 1  # (it re-runs sweeps of its own)
+        assert back["kernel_launches"] == general["kernel_launches"] + RESIDENT_LAUNCHES
+        assert rel_err(got["P"], ref["P"]) <= PARITY_TOL
+    else:
+        assert back["kernel_launches"] > RESIDENT_LAUNCHES and back["fallback_events"] == 1
+    assert rel_err(got["P"], ORACLE[method](a, b, C, 0.1, max_iter=12, zero_tol=0.0)["P"]) <= PARITY_TOL
