@@ -729,27 +729,33 @@ int sinkhorn_device(Context* ctx, cudaStream_t st, bool vanilla, double* P, doub
   // Problems that fit on the chip run in one launch.  The log method asks for
   // the scaling form with its default absorption bound; a problem that leaves
   // the form's range comes back here and starts again.
-  int launches = 0;  // those of a solve that comes back count
+  ResidentTry resident;
   if (vanilla || (option("log_sinkhorn.scaled", 1.0) != 0.0 && option("log_sinkhorn.tau", 100.0) >= 100.0)) {
-    int status = 0;
     const int rc = sinkhorn_resident(ctx, st, vanilla, P, want_grad ? grad_a : nullptr, f, g, loss, iter, err, a, b, C,
-                                     M, N, reg, max_iter, zero_tol, &status, &launches);
+                                     M, N, reg, max_iter, zero_tol, &resident);
     if (rc < 0) return rc;
-    if (rc > 0) return status;
+    if (rc > 0) return resident.status;
   }
-  const bool handed_back = launches > 0;
+  const bool handed_back = resident.launches > 0;
+  int launches = resident.launches;
 
-  // support reduction (src/sinkhorn_impl_log.cpp:238-249): drop zero masses
-  std::vector<double> ha(M), hb(N);
-  RWIG_CUDA_TRY(cudaMemcpyAsync(ha.data(), a, sizeof(double) * M, cudaMemcpyDeviceToHost, st));
-  RWIG_CUDA_TRY(cudaMemcpyAsync(hb.data(), b, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
-  RWIG_CUDA_TRY(cudaStreamSynchronize(st));
+  // support reduction (src/sinkhorn_impl_log.cpp:238-249): drop zero masses.  A
+  // call that was handed back knows their number, and needs no copy when it is
+  // zero (of 50 us that the attempt adds to a call, the copies take 20).
   std::vector<int> ri, ci;
-  for (int i = 0; i < M; ++i)
-    if (ha[i] != 0.0) ri.push_back(i);
-  for (int j = 0; j < N; ++j)
-    if (hb[j] != 0.0) ci.push_back(j);
-  const int m = (int)ri.size(), n = (int)ci.size();
+  int m = M, n = N;
+  if (!(handed_back && resident.support_m == M && resident.support_n == N)) {
+    std::vector<double> ha(M), hb(N);
+    RWIG_CUDA_TRY(cudaMemcpyAsync(ha.data(), a, sizeof(double) * M, cudaMemcpyDeviceToHost, st));
+    RWIG_CUDA_TRY(cudaMemcpyAsync(hb.data(), b, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
+    RWIG_CUDA_TRY(cudaStreamSynchronize(st));
+    for (int i = 0; i < M; ++i)
+      if (ha[i] != 0.0) ri.push_back(i);
+    for (int j = 0; j < N; ++j)
+      if (hb[j] != 0.0) ci.push_back(j);
+    m = (int)ri.size();
+    n = (int)ci.size();
+  }
   if (m == 0 || n == 0)
     return set_error(RWIG_E_INVALID, "a and b must each have at least one non-zero entry");
   if (m > 8192) return set_error(RWIG_E_UNSUPPORTED, "more than 8192 supported rows");

@@ -222,6 +222,10 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
   double* const rowp = colp + (size_t)p.chunks * ldn;
   double* const es = rowp + 1024;
 
+  if (cta == 0 && tid == 0) {
+    p.res[kResSupM] = p.info[0];
+    p.res[kResSupN] = p.info[1];
+  }
   if (p.info[2] != 0.0) {  // a mass the scaling form does not take, or no support
     if (cta == 0 && tid == 0) p.res[kResStatus] = kResUnsafe;
     return;
@@ -251,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
     const int dc = NTT / mr, di = NTT - dc * mr;
     int c = tid / mr, i = tid - c * mr;
     const double* const Cb = p.C + (size_t)n0 * M + m0;
-    while (c < ns) {
+    while (c < ns && !bad) {  // (what a thread that found K out of range leaves out is not used)
       double x[4];
       int cc[4], ii[4];
 #pragma unroll
@@ -415,7 +419,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
     for (int k = 1;; ++k) {  // loop k: u_k is in su, u_{k-1} in suo, the terms of v_{k-1} in sd
       errors_wait();
       if (es[2] != 0.0) return;
-      const unsigned long long now = p.epoch + k, last = now - 1;
+      const unsigned long long now = p.epoch + k, from = k == 1 ? now : now - 1;
       double e = 0.0, ec = 0.0;
       for (int i = ea + lane; i < eb; i += 32) {
         const double a = sa[i], x = su[i];
@@ -433,11 +437,13 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
       if (k == 1 && es[3] != 0.0) e = INFINITY;  // K has subnormal entries
       if (lane < 2) put(error_at(now) + 2 * cta + lane, lane ? ec : e, now);
       double verdict = 0.0, er = 0.0;
-      if (k > 1) {  // iteration k - 2 (of iteration 0: the range checks)
+      // loop 1 waits for its own exchange (the checks of K and of the first u, so
+      // that a problem out of range leaves early), loop k > 2 judges iteration k - 2
+      if (k != 2) {
         constexpr int NP = 2 * kMaxG / 32;
         double x[NP], t[2] = {0.0, 0.0};
         const int n = (G - lane + 31) >> 5;
-        const bool ok = poll<NP>(2 * n, [&](int q) { return error_at(last) + 2 * (lane + 32 * (q >> 1)) + (q & 1); }, last, x, p.err);
+        const bool ok = poll<NP>(2 * n, [&](int q) { return error_at(from) + 2 * (lane + 32 * (q >> 1)) + (q & 1); }, from, x, p.err);
 #pragma unroll
         for (int q = 0; q < NP; ++q) t[q & 1] += x[q];
         const double e0 = warp_sum(t[0]), e1 = warp_sum(t[1]);
@@ -596,8 +602,6 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
           p.res[kResL1Col] = es[4];
           p.res[kResL2Row] = sqrt(es[7]);
           p.res[kResL2Col] = sqrt(es[5]);
-          p.res[kResSupM] = p.info[0];
-          p.res[kResSupN] = p.info[1];
           p.res[kResGradNs] = 0.0;
         }
       }
@@ -757,7 +761,7 @@ enum { SRS_PACKETS = 250, SRS_INFO };
 
 int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, double* grad_a, double* f, double* g,
                       double* loss, int* iter, double* err, const double* a, const double* b, const double* C, int M,
-                      int N, double reg, int max_iter, double zero_tol, int* status_out, int* launches) {
+                      int N, double reg, int max_iter, double zero_tol, ResidentTry* out) {
   using namespace skres;
   const bool grad = grad_a != nullptr;
   Shape s;
@@ -822,11 +826,13 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   if (grad) rc = s.reg ? launch<true, true>(ctx, p, s, st) : launch<true, false>(ctx, p, s, st);
   else rc = s.reg ? launch<false, true>(ctx, p, s, st) : launch<false, false>(ctx, p, s, st);
   if (rc) return rc;
-  *launches = 2;
+  out->launches = 2;
   RWIG_CUDA_TRY(cudaEventRecord(ctx->ev1, st));
   RWIG_CUDA_TRY(cudaEventSynchronize(ctx->ev1));
   const int outcome = words_outcome(res);
   if (outcome < 0) return set_error(RWIG_E_TIMEOUT, "Sinkhorn kernel stopped by a bounded wait");
+  out->support_m = (int)res[kResSupM];
+  out->support_n = (int)res[kResSupN];
   if (outcome == 0) return 0;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
@@ -835,10 +841,10 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   if (loss) *loss = res[kResLoss];
   if (iter) *iter = it;
   if (err) *err = e;
-  *status_out = (e <= zero_tol) ? 0 : (it == max_iter ? 1 : 2);
+  out->status = (e <= zero_tol) ? 0 : (it == max_iter ? 1 : 2);
   rwig_report& R = report();
   R.iter = it;
-  R.status = *status_out;
+  R.status = out->status;
   R.err = e;
   R.marg_l1_row = res[kResL1Row];
   R.marg_l1_col = res[kResL1Col];
@@ -849,9 +855,9 @@ int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, do
   R.grad_ms = res[kResGradNs] * 1e-6;
   R.sweep_ms = ms - R.grad_ms;
   R.sweep_iters = it;
-  R.kernel_launches = *launches;
-  R.support_m = (int)res[kResSupM];
-  R.support_n = (int)res[kResSupN];
+  R.kernel_launches = out->launches;
+  R.support_m = out->support_m;
+  R.support_n = out->support_n;
   return 1;
 }
 

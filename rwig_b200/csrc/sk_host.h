@@ -62,13 +62,19 @@ int sinkhorn_grad(Context* ctx, cudaStream_t st, bool vanilla, const double* C, 
 constexpr int kSlotHistoryF = 31, kSlotHistoryG = 32;
 constexpr size_t kMaxHistoryBytes = size_t(32) << 30;
 
+// What a solve in one launch leaves its caller: the reference status when it
+// finished; else the kernels that ran from event ev0 on (none when the problem
+// does not fit) and, if any did, the non-zero masses of either side.
+struct ResidentTry {
+  int status = 0, launches = 0, support_m = 0, support_n = 0;
+};
+
 // A whole solve in one launch (sinkhorn_resident.cu), grad_a optional: 1 with
-// *status and the report filled, 0 when the problem does not fit or left the
-// scaling form's range (nothing of its outputs is to be used; *launches counts
-// what ran from event ev0 on, none when it does not fit), < 0 an error.
+// the report filled, 0 when the problem does not fit or left the scaling form's
+// range (nothing of its outputs is to be used), < 0 an error.
 int sinkhorn_resident(Context* ctx, cudaStream_t st, bool vanilla, double* P, double* grad_a, double* f, double* g,
                       double* loss, int* iter, double* err, const double* a, const double* b, const double* C, int M,
-                      int N, double reg, int max_iter, double zero_tol, int* status, int* launches);
+                      int N, double reg, int max_iter, double zero_tol, ResidentTry* out);
 
 int sinkhorn_device(Context* ctx, cudaStream_t st, bool vanilla, double* P, double* grad_a, double* f, double* g,
                     double* loss, int* iter, double* err, const double* a, const double* b, const double* C,

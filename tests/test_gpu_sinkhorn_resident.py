@@ -158,3 +158,33 @@ def test_report_of_a_handed_back_call(method):
     else:
         assert back["kernel_launches"] > RESIDENT_LAUNCHES and back["fallback_events"] == 1
     assert rel_err(got["P"], ORACLE[method](a, b, C, 0.1, max_iter=12, zero_tol=0.0)["P"]) <= PARITY_TOL
+
+
+# subnormal entries of K; a plan that underflows from the first iterations on, and
+# one that does so on zero entries of K only; a mass whose scaling is out of range;
+# a negative one
+@pytest.mark.parametrize("m,n,method,reg,mass,zeros", [
+    (90, 70, "log", 1e-3, None, False), (481, 300, "log", 1e-3, None, True), (90, 70, "vanilla", 1.2e-3, None, False),
+    (200, 300, "vanilla", 1e-3, None, True), (90, 70, "vanilla", 5e-4, None, False), (90, 70, "log", 0.1, 1e-280, True),
+    (90, 70, "vanilla", 0.1, 1e-280, False),
+])
+@pytest.mark.parametrize("max_iter", [1, 2, 3, 25])
+def test_handed_back_early(m, n, method, reg, mass, zeros, max_iter):
+    """Calls that leave the scaling form in the first iterations or have no
+    finite gradient, with full and with reduced supports."""
+    a, b, C = _problem(m, n, zeros)
+    if mass:
+        a[1] = mass
+    par = {"reg": reg, "method": method, "with_grad": True, "max_iter": max_iter, "zero_tol": 0.0}
+    got = rw.sinkhorn(a, b, C, par)
+    rep = rw.last_report()
+    assert rep["fallback_events"] >= 1 and rep["kernel_launches"] > RESIDENT_LAUNCHES
+    assert rep["support_m"] == int((a != 0).sum()) and rep["support_n"] == int((b != 0).sum())
+    ref = ORACLE[method](a, b, C, reg, with_grad=True, max_iter=max_iter, zero_tol=0.0)
+    assert got["iter"] == ref["iter"] == max_iter
+    assert rel_err(got["P"], ref["P"]) <= PARITY_TOL
+    x, y = ("f", "g") if method == "log" else ("u", "v")
+    sc = dual_scale(ref[x], ref[y]) if method == "log" else None
+    assert rel_err(got[x], ref[x], sc) <= PARITY_TOL and rel_err(got[y], ref[y], sc) <= PARITY_TOL
+    if method == "log":
+        assert rel_err(got["grad_a"], ref["grad_a"]) <= PARITY_TOL
