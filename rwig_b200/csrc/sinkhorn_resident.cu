@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
       if (kind == 0) {
         const double x = exp(-c / eps);
         if (!p.vanilla && !(x >= 2.2250738585072014e-308 && x <= 1.79e308)) bad = true;
+        if (GRAD) zero_plan |= x < 1e-250;
         return x;
       }
       if (sa[i] == 0.0 || sb[j] == 0.0) return 0.0;
@@ -414,6 +415,27 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
 
   // ---------------------------------------------------------------- error warp
   if (w == NW) {
+    // Gradient: whether an entry of the plan u_i K_ij v_j of its block is below half
+    // of the smallest subnormal number.  A plan with such an entry has no finite
+    // gradient and the call is the general drivers' (which repeat the reference's
+    // NaN).  The plan itself is the test that counts, but finding it there costs the
+    // whole forward: 1270 us of the general drivers became 1617 at 701 x 513, 50
+    // iterations; found after two iterations, on blocks with entries of K below
+    // 1e-250, 1293.
+    auto underflows = [&]() {
+      auto ex = [](double x) { return __double2hiint(x) >> 20; };  // (biased)
+      int low = 0;
+      for (int i = lane; i < mr; i += 32) {
+        const int eu = su[i] != 0.0 ? ex(su[i]) - 3 * 1023 : 0x10000;
+#pragma unroll 8
+        for (int c = 0; c < ns; ++c) {
+          const double x = K[(size_t)c * lds + i];
+          const int ev = ex(sv[c]);
+          low = min(low, eu + (x != 0.0 ? ex(x) : -1076 + 1023) + (ev ? ev : 0x10000));
+        }
+      }
+      return __any_sync(0xffffffffu, low < -1077);
+    };
     // this CTA's share: rows and columns of its block's row and column
     const int ea = ci * mr / gc, eb = (ci + 1) * mr / gc, ec0 = ri * nr / gr, ec1 = (ri + 1) * nr / gr;
     for (int k = 1;; ++k) {  // loop k: u_k is in su, u_{k-1} in suo, the terms of v_{k-1} in sd
@@ -435,6 +457,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
       e = warp_sum(e);
       ec = warp_sum(ec);
       if (k == 1 && es[3] != 0.0) e = INFINITY;  // K has subnormal entries
+      if (GRAD && k == 3 && es[4] != 0.0 && underflows()) e = INFINITY;  // (of u_3, v_2)
       if (lane < 2) put(error_at(now) + 2 * cta + lane, lane ? ec : e, now);
       double verdict = 0.0, er = 0.0;
       // loop 1 waits for its own exchange (the checks of K and of the first u, so
@@ -478,6 +501,8 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
       fill(kind);
       const bool any = sync_or(bad);
       if (stage == kInit) {
+        const bool look = GRAD && sync_or(zero_plan);
+        zero_plan = false;
         if (tid < nr) {
           sv[tid] = b_j != 0.0 ? 1.0 : 0.0;  // K 1 over the support
           sd[tid] = 0.0;
@@ -485,6 +510,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
         if (tid == 0) {
           es[1] = es[2] = 0.0;
           es[3] = any ? 1.0 : 0.0;
+          es[4] = look ? 1.0 : 0.0;
         }
       } else if (stage == kBackward0) {
         if (tid < nr) sv[tid] = b_j != 0.0 ? s * v * rb_j : 0.0;
