@@ -35,7 +35,7 @@
 // 26 of them per exponential, 14 in FP64): 2048 x 2048 x 32 takes 355 us a pass.
 // Small ones are bound by one CTA's chain (two loads from L2, the exponentials,
 // two warp reductions, log: 3 us) and the launch: programmatic launches let the
-// next pass's CTAs stand by.  360 x 360 x 5, 20 iterations with gradient: 640 us
+// next pass's CTAs stand by.  360 x 360 x 5, 20 iterations with gradient: 650 us
 // a call, 7.5 us a pass; with 64 x 16 output tiles and slices of the reduction
 // axis merged by another kernel, 18 CTAs in all there, it took 6047 us, and 8039
 // against 7144 us for 5 iterations of 2048 x 2048 x 32.

@@ -62,7 +62,7 @@ struct GemmArgs {
   int tcols;         // output columns per tile (<= BN; 0: BN).  A multiple of an
                      // epilogue's column group keeps every group inside one tile.
   int tile0;         // first tile of the launch (wide-tile kernel; 0 otherwise)
-  int early;         // K was not written by the kernel before this one in the stream (see gemm)
+  int early;         // K's tiles may be read before the products in flight end (see load_first)
 };
 
 template <int TRANS>
@@ -232,7 +232,11 @@ __device__ __forceinline__ void load_stage(const GemmArgs& g, double* As, double
 }
 // The first STG - 1 stages.  The next product of the stream may start while
 // this one drains; it reads nothing written by the kernel before it until that
-// has ended, but K's tiles on `early`.
+// has ended, but K's tiles on `early`.  A product lets its dependents start
+// before its own wait, so behind a chain of products an early read can come
+// before the end of any of them: it is safe only when K's writer is followed by
+// at least one ordinary launch (which starts after the writer's end, and lets the
+// first product start at its own end).
 template <int TRANS, int NT, int XV, int BMT, int STG, int ASZ, int BSZ>
 __device__ __forceinline__ void load_first(const GemmArgs& g, double* As, double* Bs, int m0, int n0, int tc,
                                            int kbeg, int kend, int nsteps) {
@@ -528,10 +532,12 @@ struct EpiStore {
 // host side
 // ---------------------------------------------------------------------------
 // Largest power of two <= kMaxSplits that keeps the grid within about the
-// resident CTAs of one wave (two per SM for NT = 4, one for NT = 8) and
-// leaves every slice a BK step: a split divides the epilogue's rows too, and at
-// small sizes that is what counts.  A 200-word, 64-column gradient of 80 products
-// took 2500 us unsplit (slices of at least four steps) and takes 605 us in eight.
+// resident CTAs of one wave (two per SM for NT = 4, one for NT = 8) while the
+// slices before the last doubling have a BK step each.  Up to half the slices
+// may so be empty: their CTAs have no contraction, but a split divides the
+// epilogue's rows too, and at small sizes that is what counts.  A 200-word,
+// 64-column gradient of 80 products took 2500 us unsplit (slices of at least four
+// steps) and takes 592 us in eight.
 inline int pick_splits(const Context* ctx, int Mo, int Kd, int W, int NT, int tc = 0) {
   if (tc <= 0) tc = NT * 8;
   const long long tiles = (long long)((Mo + BM - 1) / BM) * ((W + tc - 1) / tc);

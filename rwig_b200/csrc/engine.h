@@ -52,11 +52,11 @@ struct Context {
   // whole-solve Sinkhorn launches (sinkhorn_resident.cu): host-mapped results
   // and the number of the last launch, which its packets' tags carry
   double* resident_res = nullptr;
+  unsigned long long resident_epoch = 0;
   // host-mapped words through which kernels of the barycenter and WDL paths
   // tell a waiting or enqueuing host what it must know (allocated on first use)
   static constexpr int kMappedWords = 2 + 64 * 64;
   double* mapped = nullptr;
-  unsigned long long resident_epoch = 0;
   // dynamic shared memory each kernel may use on this device (raise_smem)
   std::map<const void*, size_t> smem_raised;
   // clusters of each size that can be resident at once, by kernel (dgemm.cuh; 0
@@ -99,8 +99,10 @@ void gemm_timer_end(Context* ctx, double* ms, int* launches);
 // device: a process that uses several raises it on each.
 int raise_smem(Context* ctx, const void* kern, size_t bytes);
 
+// Allocates Context::mapped; 0 or an engine error code.
+int ensure_mapped(Context* ctx);
+
 // Grow-only scratch slot `k` of at least `bytes`; nullptr on failure.
-int ensure_mapped(Context* ctx);  // Context::mapped; 0 or an engine error code
 void* scratch(Context* ctx, int k, size_t bytes);
 
 // Engine options (rwig_set_option); unknown names return `dflt`.

@@ -10,8 +10,12 @@
 // marginals from C at the end.  Zero masses need no packing: their scalings are
 // zero and drop out of every sum.  The solve is given up (status kResUnsafe,
 // and the general drivers in sinkhorn_log.cu start again from scratch) when a
-// mass is negative or not finite, when K has subnormal entries (log method), or
-// when a sum or a scaling leaves the safe range, or the gradient is not finite.
+// mass is negative or not finite, when K has subnormal entries (log method),
+// when a sum or a scaling leaves the safe range or, with a gradient, when a plan
+// entry underflows or the gradient is not finite.  K and the first u are judged
+// within the first iteration: 20 log iterations that are given up there take 485
+// us at 701 x 513, 470 in the general drivers alone.  A scaling that leaves the
+// range later (only with max C / eps above 575) costs the iterations up to there.
 //
 // The gradient with respect to a (Sinkhorn::_bwd_vanilla :169-213, _bwd_log
 // :379-520: one function, so one gradient) is unrolled in the same launch from
@@ -38,11 +42,13 @@
 //     launch's number and the round, so packets need no reset;
 //   * 15 warps iterate; the last one only forms, exchanges and judges the
 //     stopping error, two iterations behind (what was computed since is thrown
-//     away when it stops).
+//     away when it stops);
+//   * a gradient's scalings are stored once, by the first CTA of each block row
+//     and column, and read back from L2 behind one fence.
 // Whole solves through the C entry against the general drivers (us): 256 x 256
-// vanilla, 19 iterations 135 (430); 1777 x 1501 log, 31 iterations 328 (723);
-// with gradient 701 x 513 vanilla, 11 iterations 202 (482); 2048 x 2048 log,
-// 100 iterations 1980 (5326), 9.5 us per iteration in each direction: of about
+// vanilla, 19 iterations 134 (430); 1777 x 1501 log, 31 iterations 324 (723);
+// with gradient 701 x 513 vanilla, 11 iterations 192 (482); 2048 x 2048 log,
+// 100 iterations 1972 (5326), 9.5 us per iteration in each direction: of about
 // 17500 clocks the two passes take 6600, the exchanges 4000-5000 each.
 #include <algorithm>
 #include <cmath>
