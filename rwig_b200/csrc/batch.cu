@@ -1275,7 +1275,8 @@ void bind(batch::Prob& d, double* k, double* w, double* res, unsigned* ctl) {
 int launch_service(Context* ctx, cudaStream_t st, const batch::Prob* dprob, const unsigned* pub, unsigned* done,
                    unsigned* dctl, double* dprof, unsigned long long idle_ns, unsigned avail0, unsigned head0) {
   using namespace batch;
-  if (int rc = raise_smem(ctx, (const void*)service_kernel, smem_bytes())) return rc;
+  static const KernelSlot slot;
+  if (int rc = raise_smem(ctx, slot, (const void*)service_kernel, smem_bytes())) return rc;
   int nblk = 0;
   RWIG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nblk, service_kernel, NTT, smem_bytes()));
   if (nblk < 1) return set_error(RWIG_E_UNSUPPORTED, "batched Sinkhorn kernel does not fit on an SM");

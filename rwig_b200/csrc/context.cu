@@ -173,11 +173,15 @@ void* scratch(Context* ctx, int k, size_t bytes) {
   return p;
 }
 
-int raise_smem(Context* ctx, const void* kern, size_t bytes) {
-  size_t& have = ctx->smem_raised[kern];
-  if (have >= bytes) return 0;
+KernelSlot::KernelSlot() : index([] {
+  static std::atomic<int> count{0};
+  return count.fetch_add(1);
+}()) {}
+
+int raise_smem_first(Context* ctx, const KernelSlot& slot, const void* kern, size_t bytes) {
+  if (ctx->smem_raised.size() <= (size_t)slot.index) ctx->smem_raised.resize(slot.index + 1, 0);
   RWIG_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  have = bytes;
+  ctx->smem_raised[slot.index] = bytes;
   return 0;
 }
 

@@ -553,7 +553,8 @@ template <int TRANS, int NT, int XV, class Epi, int KM>
 int launch_kernel(Context* ctx, const GemmArgs& g, const Epi& epi, cudaStream_t st) {
   constexpr size_t bytes = sizeof(double) * smem_doubles<TRANS, NT>();
   auto kern = dgemm_kernel<TRANS, NT, XV, Epi, KM>;
-  if (int rc = raise_smem(ctx, (const void*)kern, bytes)) return rc;
+  static const KernelSlot slot;
+  if (int rc = raise_smem(ctx, slot, (const void*)kern, bytes)) return rc;
   cudaLaunchConfig_t cfg = {};
   const int tc = g.tcols > 0 ? g.tcols : NT * 8;
   cfg.gridDim = dim3((unsigned)(((g.Mo + BM - 1) / BM) * ((g.W + tc - 1) / tc)), 1, g.splits);
@@ -574,10 +575,16 @@ int launch_kernel(Context* ctx, const GemmArgs& g, const Epi& epi, cudaStream_t 
 }
 
 template <int TRANS, int XV, class Epi, int KM>
+const KernelSlot& kernel2_slot() {
+  static const KernelSlot slot;
+  return slot;
+}
+
+template <int TRANS, int XV, class Epi, int KM>
 int prepare_kernel2(Context* ctx) {
   constexpr size_t bytes = sizeof(double) * smem2_doubles<TRANS>();
   static_assert(bytes <= 227 * 1024, "wide-tile GEMM exceeds the shared memory of a CTA");
-  return raise_smem(ctx, (const void*)dgemm2_kernel<TRANS, XV, Epi, KM>, bytes);
+  return raise_smem(ctx, kernel2_slot<TRANS, XV, Epi, KM>(), (const void*)dgemm2_kernel<TRANS, XV, Epi, KM>, bytes);
 }
 
 // Clusters of `s` wide-tile CTAs that can be resident at once (cached per
@@ -585,7 +592,7 @@ int prepare_kernel2(Context* ctx) {
 template <int TRANS, int XV, class Epi, int KM>
 int max_clusters2(Context* ctx, int s) {
   static_assert(kMaxSplits < Context::kClusterSizes, "cluster sizes of the cache");
-  int* const cache = ctx->clusters[(const void*)dgemm2_kernel<TRANS, XV, Epi, KM>].data();
+  int* const cache = ctx->clusters[kernel2_slot<TRANS, XV, Epi, KM>().index].data();
   if (cache[s] == 0) {
     if (prepare_kernel2<TRANS, XV, Epi, KM>(ctx) != 0) return 0;
     cudaLaunchConfig_t cfg = {};

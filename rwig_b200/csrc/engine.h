@@ -15,6 +15,14 @@
 
 namespace rwig {
 
+// A kernel's place in the tables of Context that are kept per kernel: one static
+// object beside each launch.  (Found by its address in a map instead, a kernel's
+// limit cost 0.2 us a launch, 0.7% of a WDL training call.)
+struct KernelSlot {
+  const int index;
+  KernelSlot();
+};
+
 // A captured launch sequence, replayed when a call repeats with the same
 // arguments and buffers (key).
 struct GraphEntry {
@@ -58,11 +66,11 @@ struct Context {
   static constexpr int kMappedWords = 2 + 64 * 64;
   double* mapped = nullptr;
   // dynamic shared memory each kernel may use on this device (raise_smem)
-  std::map<const void*, size_t> smem_raised;
+  std::vector<size_t> smem_raised;  // by KernelSlot::index
   // clusters of each size that can be resident at once, by kernel (dgemm.cuh; 0
   // not asked, -1 none)
   static constexpr int kClusterSizes = 9;
-  std::map<const void*, std::array<int, kClusterSizes>> clusters;
+  std::map<int, std::array<int, kClusterSizes>> clusters;  // by KernelSlot::index
   // the K whose INT8 residue planes the scratch holds (oz::prepare_reuse):
   // its size and leading dimension, valid while no other prepare ran
   bool oz_kept = false;
@@ -97,7 +105,11 @@ void gemm_timer_end(Context* ctx, double* ms, int* launches);
 // Lets `kern` use `bytes` of dynamic shared memory on the context's device, which
 // is current; 0 or an engine error code.  The limit belongs to a kernel on one
 // device: a process that uses several raises it on each.
-int raise_smem(Context* ctx, const void* kern, size_t bytes);
+int raise_smem_first(Context* ctx, const KernelSlot& slot, const void* kern, size_t bytes);
+inline int raise_smem(Context* ctx, const KernelSlot& slot, const void* kern, size_t bytes) {
+  if ((size_t)slot.index < ctx->smem_raised.size() && ctx->smem_raised[slot.index] >= bytes) return 0;
+  return raise_smem_first(ctx, slot, kern, bytes);
+}
 
 // Allocates Context::mapped; 0 or an engine error code.
 int ensure_mapped(Context* ctx);

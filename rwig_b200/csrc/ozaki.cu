@@ -616,10 +616,12 @@ int launch_i8(Context* ctx, const int8_t* A, int Mpad, const int8_t* B, int Wpad
   const int grid = std::min(tiles, ctx->sm_count);  // persistent: one CTA per SM
   const bool timed = gemm_timer_mark(ctx, st);
   if (MT == 256) {
-    if (int rc = raise_smem(ctx, (const void*)i8_gemm<RAW, 256>, kGemmSmem)) return rc;
+    static const KernelSlot slot;
+    if (int rc = raise_smem(ctx, slot, (const void*)i8_gemm<RAW, 256>, kGemmSmem)) return rc;
     i8_gemm<RAW, 256><<<grid, kPersistThreads, kGemmSmem, st>>>(ta, tb, g, ntn, ntm, planes);
   } else {
-    if (int rc = raise_smem(ctx, (const void*)i8_gemm<RAW, 128>, kGemmSmem)) return rc;
+    static const KernelSlot slot;
+    if (int rc = raise_smem(ctx, slot, (const void*)i8_gemm<RAW, 128>, kGemmSmem)) return rc;
     i8_gemm<RAW, 128><<<grid, kPersistThreads, kGemmSmem, st>>>(ta, tb, g, ntn, ntm, planes);
   }
   RWIG_CUDA_TRY(cudaGetLastError());

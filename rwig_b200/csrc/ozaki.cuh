@@ -232,7 +232,8 @@ int gemm(Context* ctx, const Prepared& pr, int trans, const double* X, long long
   if (int rc = products(ctx, pr, trans, X, ldx, W, st, &cres, &beta, &Wpad, launches, lane)) return rc;
   if (tc <= 0 || tc > kCrtCols) tc = kCrtCols;
   const size_t smem = epi_smem_bytes();
-  if (int rc = raise_smem(ctx, (const void*)crt_tiles<Epi>, smem)) return rc;
+  static const KernelSlot slot;
+  if (int rc = raise_smem(ctx, slot, (const void*)crt_tiles<Epi>, smem)) return rc;
   const dim3 grid((pr.Mo + kCrtRows - 1) / kCrtRows, (W + tc - 1) / tc);
   crt_tiles<Epi><<<grid, kCrtThreads, smem, st>>>(crt_constants(), cres, pr.Mpad, Wpad, row_exponents(pr, trans), beta,
                                                    pr.Mo, W, tc, epi);

@@ -781,7 +781,8 @@ bool shape(const Context* ctx, int M, int N, Shape* best) {
 template <bool GRAD, bool REG>
 int launch(Context* ctx, Args& p, const Shape& s, cudaStream_t st) {
   auto kern = resident_kernel<GRAD, REG>;
-  if (int rc = raise_smem(ctx, (const void*)kern, s.smem)) return rc;
+  static const KernelSlot slot;
+  if (int rc = raise_smem(ctx, slot, (const void*)kern, s.smem)) return rc;
   void* args[] = {&p};
   RWIG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)kern, dim3(s.gr * s.gc), dim3(kThreads), args, s.smem, st));
   return 0;

@@ -54,6 +54,7 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 
 int main() {
   static int kern, other;
+  static const rwig::KernelSlot ks, os;
   rwig::Context* ctx[2];
   for (int d = 0; d < 2; ++d) {
     CHECK(rwig_init(d) == 0);
@@ -63,12 +64,12 @@ int main() {
   CHECK(ctx[0] != ctx[1]);
   for (int d = 0; d < 2; ++d) {  // the same kernel on either device, small launches after large ones
     cudaSetDevice(d);
-    CHECK(rwig::raise_smem(ctx[d], &kern, 200000) == 0 && g_limit[std::make_pair(d, &kern)] == 200000);
-    CHECK(rwig::raise_smem(ctx[d], &kern, 60000) == 0 && g_limit[std::make_pair(d, &kern)] == 200000);
-    CHECK(rwig::raise_smem(ctx[d], &other, 60000) == 0 && g_limit[std::make_pair(d, &other)] == 60000);
+    CHECK(rwig::raise_smem(ctx[d], ks, &kern, 200000) == 0 && g_limit[std::make_pair(d, &kern)] == 200000);
+    CHECK(rwig::raise_smem(ctx[d], ks, &kern, 60000) == 0 && g_limit[std::make_pair(d, &kern)] == 200000);
+    CHECK(rwig::raise_smem(ctx[d], os, &other, 60000) == 0 && g_limit[std::make_pair(d, &other)] == 60000);
     CHECK(g_calls == 2 * (d + 1));
   }
-  CHECK(rwig::raise_smem(ctx[1], &kern, 210000) == 0 && g_limit[std::make_pair(1, &kern)] == 210000 && g_calls == 5);
+  CHECK(rwig::raise_smem(ctx[1], ks, &kern, 210000) == 0 && g_limit[std::make_pair(1, &kern)] == 210000 && g_calls == 5);
   rwig_shutdown();
   return 0;
 }
