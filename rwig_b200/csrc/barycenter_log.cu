@@ -55,6 +55,10 @@ namespace barylog {
 constexpr int kMaxWarps = 16;  // per CTA
 constexpr int kChunk = 4;      // reduction elements a lane holds at once
 constexpr int kSpread = 4;     // replicas of the exponential's table
+// Where a maximum starts.  Finite, so that a lane or a warp whose every term is
+// exp(-inf) (zero masses, infinite costs) keeps a sum of zero, which adds nothing
+// to the others' (from -inf on it is 0 * exp(-inf + inf) = NaN).
+constexpr double kNoTerm = -1.7976931348623157e308;
 
 enum Mode { kColFwd, kRowFwd, kColBwd, kRowBwd };
 
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2) pass_kernel(Pass a) {
         P[q] = a.P + (size_t)s * K;
         Y[q] = FWD ? nullptr : a.Y + (size_t)s * K;
         qv[q] = FWD ? 0.0 : a.Q[o + (size_t)s * O] * ie;
-        mx[q] = -INFINITY;
+        mx[q] = kNoTerm;
         sm[q] = 0.0;
       }
       for (int kb = 32 * ki; kb < K; kb += CH * step) {
@@ -184,9 +188,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2) pass_kernel(Pass a) {
         }
         t = warp_sum(t);
         if (lane == 0 && s0 + q < S) {
-          // a warp whose every term is exp(-inf) (zero masses, infinite costs),
-          // 0 * NaN here, adds nothing to the other warps' terms
-          part[ki * S + s0 + q] = FWD && m == -INFINITY && a.kw > 1 ? 0.0 : t;
+          part[ki * S + s0 + q] = t;
           if (FWD) part[(a.kw + ki) * S + s0 + q] = m;
         }
       }
@@ -201,12 +203,12 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2) pass_kernel(Pass a) {
       for (int s = tid; s < S; s += ns) {
         double t = 0.0;
         if (FWD) {
-          double m = -INFINITY;
+          double m = kNoTerm;
           for (int z = 0; z < a.kw; ++z) m = fmax(m, part[(a.kw + z) * S + s]);
           if (a.kw == 1) t = part[s];
           else
             for (int z = 0; z < a.kw; ++z) t += part[z * S + s] * exp(part[(a.kw + z) * S + s] - m);
-          t = -a.eps * (m + log(t));
+          t = -a.eps * (m + log(t == 0.0 ? NAN : t));  // (an output without a finite term)
         } else {
           for (int z = 0; z < a.kw; ++z) t += part[z * S + s];
         }
