@@ -130,6 +130,13 @@ __device__ __forceinline__ void get(const Packet* p, unsigned long long& v, unsi
                : "memory");
 }
 
+// 8 bytes to shared memory, no register held meanwhile; the thread waits for its own.
+__device__ __forceinline__ void copy8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Polls NP packets at(k), k < n, until all carry the tag (n <= 0: none);
 // bounded (2 s, or an error elsewhere).  All loads of a try are issued before
 // the first is looked at: a test after each load would cost a round trip to L2
@@ -573,7 +580,11 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
     } else if (GRAD && stage == kBackward) {
       // one factor at a time: v_l^2 alone overflows from 1e154 on, v_l (K^T x)_j is
       // of the size of the gradient's terms
-      if (tid < nr) sv[tid] = s * vl * rb_j * vl;
+      if constexpr (REG) copies_wait();
+      if (tid < nr) {
+        if constexpr (REG) vl = sd[tid];
+        sv[tid] = s * vl * rb_j * vl;
+      }
     }
     if (sync_or(!ok)) {
       ok = false;
@@ -664,17 +675,28 @@ __global__ void __launch_bounds__(kThreads, 1) resident_kernel(Args p) {
       stage = kBackward0;
       kind = 0;
       l = iter;
-      ul = u;
+      if constexpr (!REG) ul = u;
+      else if (tid < mr) suo[tid] = u;
       sync();
     } else {  // step l: x = ubar u_l^2 / a, grad += ubar u_l / a
+      if constexpr (REG) ul = tid < mr ? suo[tid] : 0.0;
       const double q = a_i != 0.0 ? t * ul / a_i : 0.0;
       ga += q;
       --l;
       if (l == 0) break;
       if (tid < mr) su[tid] = q * ul;
-      // (from L2: plain loads of lines that other CTAs share cost 0.8% of a call)
-      ul = tid < mr && a_i != 0.0 ? __ldcg(uh + (size_t)l * M + tid) : 0.0;
-      vl = tid < nr ? __ldcg(vh + (size_t)l * N + tid) : 0.0;
+      // u_l and v_l from L2 (plain loads of lines that other CTAs share cost 0.8% of a
+      // call), into registers or, where columns of K take those, into suo and sd, which
+      // are free by now: 2048 x 2048, 100 iterations, takes 1944 us on the device so and
+      // 1973 with registers; 701 x 513, which has registers left, 181-197 us a call with
+      // them and 201-204 without
+      if constexpr (REG) {
+        if (tid < mr) copy8(suo + tid, uh + (size_t)l * M + tid);
+        if (tid < nr) copy8(sd + tid, vh + (size_t)l * N + tid);
+      } else {
+        ul = tid < mr && a_i != 0.0 ? __ldcg(uh + (size_t)l * M + tid) : 0.0;
+        vl = tid < nr ? __ldcg(vh + (size_t)l * N + tid) : 0.0;
+      }
       stage = kBackward;
       if (sync_or(!ok)) {
         ok = false;

@@ -188,3 +188,16 @@ def test_handed_back_early(m, n, method, reg, mass, zeros, max_iter):
     assert rel_err(got[x], ref[x], sc) <= PARITY_TOL and rel_err(got[y], ref[y], sc) <= PARITY_TOL
     if method == "log":
         assert rel_err(got["grad_a"], ref["grad_a"]) <= PARITY_TOL
+
+
+@pytest.mark.parametrize("m,n", [(2041, 1983), (8190, 479), (600, 6700)])
+@pytest.mark.parametrize("max_iter", [1, 2, 6])
+def test_gradient_beside_register_columns(m, n, max_iter):
+    """Blocks that keep some columns of K in registers fetch the scalings of a
+    backward step into shared memory: none for one iteration, one step for two."""
+    a, b, C = _problem(m, n, True)
+    par = {"reg": 0.2, "method": "log", "with_grad": True, "max_iter": max_iter, "zero_tol": 0.0}
+    got = rw.sinkhorn(a, b, C, par)
+    assert rw.last_report()["kernel_launches"] == RESIDENT_LAUNCHES
+    ref = oracle.sinkhorn_log(a, b, C, 0.2, with_grad=True, max_iter=max_iter, zero_tol=0.0)
+    _same(got, ref, 0.2, "log")
