@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(NTT, 1) grad_kernel(Params p) {
         const int j = jb + c;
         double col;  // gbar_j (log) or z_j = (vbar_j v_j^2) / b_j (vanilla)
         if (!VAN) col = last ? cs[c] * inv_eps : -cs[c];
-        else col = ((last ? cs[c] : -cs[c]) * (gl[c] * gl[c])) / p.b[j];
+        else col = ((last ? cs[c] : -cs[c]) * gl[c]) / p.b[j] * gl[c];  // (v_j^2 alone can overflow)
 #pragma unroll
         for (int t = 0; t < RPT; ++t) {
           if (!valid[t]) continue;
@@ -206,8 +206,9 @@ __global__ void __launch_bounds__(NTT, 1) grad_kernel(Params p) {
         } else {
           const double ul = p.fh[(size_t)l * m + i];
           const double ubar = last ? T : -T;
-          p.ga[i] += (ubar * ul) / ai;           // ubar / (K v_{l-1}),  K v_{l-1} = a / u_l
-          p.xbar[i] = (ubar * (ul * ul)) / ai;   // (ubar o u_l) / (K v_{l-1}) for step l-1
+          const double q = (ubar * ul) / ai;  // ubar / (K v_{l-1}),  K v_{l-1} = a / u_l
+          p.ga[i] += q;
+          p.xbar[i] = q * ul;                 // (ubar o u_l) / (K v_{l-1}) for step l-1
         }
       }
       __syncthreads();

@@ -201,3 +201,22 @@ def test_gradient_beside_register_columns(m, n, max_iter):
     assert rw.last_report()["kernel_launches"] == RESIDENT_LAUNCHES
     ref = oracle.sinkhorn_log(a, b, C, 0.2, with_grad=True, max_iter=max_iter, zero_tol=0.0)
     _same(got, ref, 0.2, "log")
+
+
+@pytest.mark.parametrize("narrow", ["a", "b"])
+@pytest.mark.parametrize("method", ["vanilla", "log"])
+def test_gradient_of_scalings_out_of_range(method, narrow):
+    """Scalings beyond 1e250, which the general drivers take over: the squares
+    overflow there too, the gradient does not."""
+    m, n, reg = 90, 70, 0.00143
+    g = synth.rng(53, m + n)
+    x = g.random((m, 1)) * (0.1 if narrow == "a" else 1.0)
+    y = g.random((n, 1)) * (1.0 if narrow == "a" else 0.1)
+    C = (x - y.T) ** 2
+    C /= C.max()
+    a, b = synth.dirichlet(g, 1.0, m), synth.dirichlet(g, 1.0, n)
+    got = rw.sinkhorn(a, b, C, {"reg": reg, "method": method, "with_grad": True, "max_iter": 10, "zero_tol": 0.0})
+    assert rw.last_report()["fallback_events"] >= 1
+    ref = ORACLE[method](a, b, C, reg, with_grad=True, max_iter=10, zero_tol=0.0)
+    assert np.isfinite(ref["grad_a"]).all()
+    _same(got, ref, reg, method)
