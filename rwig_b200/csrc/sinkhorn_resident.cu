@@ -48,7 +48,7 @@
 // Whole solves through the C entry against the general drivers (us): 256 x 256
 // vanilla, 19 iterations 134 (430); 1777 x 1501 log, 31 iterations 324 (723);
 // with gradient 701 x 513 vanilla, 11 iterations 192 (482); 2048 x 2048 log,
-// 100 iterations 1972 (5326), 9.5 us per iteration in each direction: of about
+// 100 iterations 1929 (5332), 9.3 us per iteration in each direction: of about
 // 17500 clocks the two passes take 6600, the exchanges 4000-5000 each.
 #include <algorithm>
 #include <cmath>
@@ -766,7 +766,7 @@ int block_ld(int m) {
 // block (two passes, 16 bytes of shared memory each, at 100 B per clock) and
 // 2200 + 40 g for an exchange among g CTAs, none when a block spans the side.
 // A problem that fits on the chip always goes here: from 120 x 95 (one CTA: 237
-// us a call against 571) to 2048^2 (1980 against 5326) the general drivers lost.
+// us a call against 571) to 2048^2 (1929 against 5332) the general drivers lost.
 bool shape(const Context* ctx, int M, int N, Shape* best) {
   if (ctx->sm_count > kMaxG || M > 8192) return false;  // (the general drivers refuse more rows of support)
   double cost = 0.0;
